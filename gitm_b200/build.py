@@ -23,7 +23,7 @@ BUILD = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libgitmvert.so")
 SOURCES = ["gitm_vert.cu", "vert_adjoint.cu", "hz_kernel.cu"]
 DEPS = ["gitm_vert.cu", "vert_adjoint.cu", "hz_kernel.cu", "vert_instance.cu", "vert_instances.h", "vert_kernel.cuh",
-        "vert_ausm.cuh", "vert_adjoint.cuh", "vert_common.cuh", "vert_hz.cuh"]
+        "vert_ausm.cuh", "vert_adjoint.cuh", "vert_common.cuh", "vert_hz.cuh", "vert_math.cuh"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",

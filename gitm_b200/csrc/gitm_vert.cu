@@ -131,6 +131,8 @@ static void fill_consts(Consts& k) {
   // the six distinct DiffExp values; exp_index() in vert_kernel.cuh maps
   // each (i, j) of the DiffExp table to one of them
   const double distinct[NS] = {0.774, 0.750, 0.749, 0.710, 0.718, 0.810};
+  // Diff0 of the pairs that share each of them (one value per exponent)
+  const double d0_of[NS] = {0.969, 0.715, 3.440, 3.208, 2.939, 0.527};
   for (int s = 0; s < NS; ++s) {
     k.mass[s] = mass[s];
     k.log_mass[s] = std::log(mass[s]);
@@ -138,6 +140,7 @@ static void fill_consts(Consts& k) {
     k.k_over_m[s] = KB / mass[s];
     k.inv_vib2[s] = 1.0 / (vib[s] - 2);
     k.one_minus_e[s] = 1.0 - distinct[s];
+    k.kpair[s] = 1.0e-2 * KB / (1.0e17 * d0_of[s]);
   }
   for (int i = 0; i < NS; ++i)
     for (int j = 0; j < NS; ++j) {

@@ -700,7 +700,7 @@ __device__ inline double cell_adjoint_species(const ColCtx& c, const ColAdj& a, 
     // reciprocals on it (as friction_solve)
 #pragma unroll
     for (int p = 0; p < NS; ++p) {
-      const double ip = 1.0 / lu[p][p];
+      const double ip = rcp_nr(lu[p][p]);
       lu[p][p] = ip;
 #pragma unroll
       for (int r = p + 1; r < NS; ++r) {

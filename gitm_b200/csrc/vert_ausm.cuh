@@ -364,9 +364,13 @@ __device__ __forceinline__ void ausm_cell(ColCtx c, int i, const GitmVertParams&
   }
   // friction on the updated densities with the stage temperature (:902-913)
   if (prm.use_neutral_friction) {
-    double glc[NS];
-    grad_log_cons(c, i, glc);
-    friction_solve(dtk, nns, T, eddy, glc, wv, st);
+    friction_solve(dtk, nns, nrs, T, wv, st);
+    if (eddy != 0.0) {
+      double glc[NS];
+      grad_log_cons(c, i, glc);
+#pragma unroll
+      for (int s = 0; s < NS; ++s) wv[s] = fma(-eddy, glc[s], wv[s]);
+    }
   }
   // clamp and bulk vertical wind (:916-941)
   double NewVU = 0.0;

@@ -65,6 +65,7 @@ struct Consts {
   double inv_vib2[NS];           // 1 / (Vibration - 2)
   double kc[NS][NS];             // 1e-2 k / (Mass_i Diff0_ij): friction coefficient
   double one_minus_e[NS];        // the six distinct 1 - DiffExp values
+  double kpair[NS];              // 1e-2 k / Diff0 of each: Mass_i kc[i][j], the same for every pair of an exponent
   double log_kb;                 // log(Boltzmanns_Constant)
 };
 

@@ -21,6 +21,7 @@
 #pragma once
 
 #include "vert_common.cuh"
+#include "vert_math.cuh"
 
 namespace gv {
 
@@ -37,7 +38,8 @@ __device__ __forceinline__ int exp_index(int r, int q) {
 // ------------------------------------------------------------ smem layout
 struct Layout {
   int nAlts, G;
-  int nsl;  // slope fields in DL: 18 (Rusanov) or 32 (AUSM)
+  int P, PD;  // row pitch of the state and of the slopes
+  int nsl;    // slope fields in DL: 18 (Rusanov) or 32 (AUSM)
   int X0, XP0, X1, XP1, O, OP, OGH, DL, TU, CM, GM, SC, LT, QS, stride;
 };
 
@@ -63,6 +65,8 @@ __host__ __device__ inline Layout make_layout(int nAlts, int solver = GITM_SOLVE
   Layout L;
   L.nAlts = nAlts;
   L.G = nAlts + 4;
+  L.P = L.G;
+  L.PD = nAlts + 2;
   L.nsl = (solver == GITM_SOLVER_AUSM) ? NSLOPE_AUSM : NSTENCIL;
   const int G = L.G;
   int o = 0;
@@ -129,15 +133,15 @@ struct ColCtx {
   int xo;   // offset of the current stage buffer (X0 or X1)
   int xpo;  // offset of its passive-ion cells (XP0 or XP1)
 
-  __device__ __forceinline__ double& x(int f, int i) const { return col[xo + f * L.G + i + 1]; }
-  __device__ __forceinline__ double& o(int f, int i) const { return col[L.O + f * L.G + i + 1]; }
-  __device__ __forceinline__ double& dl(int f, int c) const { return col[L.DL + f * (L.nAlts + 2) + c]; }
+  __device__ __forceinline__ double& x(int f, int i) const { return col[xo + f * L.P + i + 1]; }
+  __device__ __forceinline__ double& o(int f, int i) const { return col[L.O + f * L.P + i + 1]; }
+  __device__ __forceinline__ double& dl(int f, int c) const { return col[L.DL + f * L.PD + c]; }
   __device__ __forceinline__ double& sc(int k) const { return col[L.SC + k]; }
   __device__ __forceinline__ double& cm(int i) const { return col[L.CM + i + 1]; }
   __device__ __forceinline__ double& tu(int i) const { return col[L.TU + i + 1]; }
   __device__ __forceinline__ double& gm(int i) const { return col[L.GM + i + 1]; }
   __device__ __forceinline__ double& ion(int s, int i) const {
-    return (s < NADV) ? col[xo + (F_I + s) * L.G + i + 1]
+    return (s < NADV) ? col[xo + (F_I + s) * L.P + i + 1]
                       : col[xpo + (s - NADV) * NPC + pcell(i, L.nAlts)];
   }
   // grid coefficient k at Fortran cell i
@@ -461,79 +465,91 @@ __device__ __forceinline__ void bc_column(ColCtx c, const GitmVertParams& prm, i
   __syncwarp();
 }
 
+// Whether ludcmp would stop on one of the rows of I + dt C (ludcmp.f:9-17: a
+// row without an element of nonzero magnitude; NaN compares false there, so a
+// row of NaN counts).  Only reached with a non-finite density or temperature.
+static __device__ __noinline__ bool friction_singular(double dt, const double* ns, const double* pw) {
+  bool singular = false;
+  for (int r = 0; r < NS; ++r) {
+    double mx = 0.0, rs = 0.0;
+    for (int q = 0; q < NS; ++q) {
+      if (q == r) continue;
+      const double dcij = c_k.kc[r][q] * (dt * ns[q]) * pw[exp_index(r, q)];
+      if (fabs(dcij) > mx) mx = fabs(dcij);
+      rs = rs + dcij;
+    }
+    if (fabs(1.0 + rs) > mx) mx = fabs(1.0 + rs);
+    singular = singular || !(mx > 0.0);
+  }
+  return singular;
+}
+
 // calc_neutral_friction (calc_neutral_friction.f90:47-106) for one cell:
-// solves (I + dt C) v = w in place and adds the eddy term -Eddy GradLogConS.
-// C_ij = 1e-2 k / (M_i D0_ij) n_j T^(1 - DiffExp_ij) (the NDensity factors of
-// the reference cancel); LU without pivoting, the matrix being strictly
-// diagonally dominant by rows for finite inputs.  ludcmp stops the run on a
-// row without an element of nonzero magnitude (ludcmp.f:9-17; NaN compares
-// false there, so a row of NaN counts): such a row sets GITM_ST_LU_SINGULAR
-// in *st (when st is given) and the solve goes on, its results non-finite.
-// A finite nonzero diagonal settles a row, so the scan of the whole row runs
-// only when the diagonal fails.
-__device__ __forceinline__ void friction_solve(double dt, const double (&ns)[NS], double T, double eddy,
-                                               const double (&glc)[NS], double (&wv)[NS],
-                                               uint32_t* st = nullptr) {
+// solves (I + dt C) v = w in place.  C_ij = 1e-2 k / (M_i D0_ij) n_j
+// T^(1 - DiffExp_ij) (the NDensity factors of the reference cancel).  Row i
+// times the species' mass density M_i n_i makes the matrix symmetric: the
+// pair coefficient 1e-2 k / D0 T^(1 - DiffExp) takes six values, one per
+// distinct exponent, and W_ij = dt (pair coefficient) n_i n_j.  With
+// S = diag(M_i n_i + sum_j W_ij) - W (diagonally dominant, so no pivoting)
+// the LDL^T elimination holds 21 values instead of 36 and takes 65
+// multiply-adds instead of 85; off the diagonal it only adds positive terms
+// (with the direct increments of rusanov_cell: the 1 degree globe's 16 steps
+// 59.3 -> 56.3 ms, error against 64-bit arithmetic 1.3e-12 -> 5e-13; the AUSM
+// solver at 2.5 degrees, 4 steps, 11.45 -> 10.60 ms).
+// mn[s] = M_s n_s.  A non-finite density or temperature takes the reference's
+// row test, which sets GITM_ST_LU_SINGULAR in *st (when st is given); the
+// solve goes on, its results non-finite.
+__device__ __forceinline__ void friction_solve(double dt, const double (&ns)[NS], const double (&mn)[NS], double T,
+                                               double (&wv)[NS], uint32_t* st = nullptr) {
   const double lt = log(T);
   double pw[NS];
 #pragma unroll
   for (int e = 0; e < NS; ++e) pw[e] = exp(c_k.one_minus_e[e] * lt);
-  // dt C_ij with dt taken into the densities once per cell: the entries
-  // -dt C_ij and the diagonal 1 + sum_j dt C_ij share each product
-  double nd[NS];
-#pragma unroll
-  for (int q = 0; q < NS; ++q) nd[q] = dt * ns[q];
-  double a[NS][NS];
-#pragma unroll
-  for (int r = 0; r < NS; ++r) {
-    double rs = 0.0;
-#pragma unroll
-    for (int q = 0; q < NS; ++q) {
-      if (q == r) continue;
-      const double dcij = c_k.kc[r][q] * nd[q] * pw[exp_index(r, q)];
-      a[r][q] = -dcij;
-      rs = rs + dcij;
-    }
-    a[r][r] = 1.0 + rs;
-  }
   if (st) {
-    bool diag_ok = true;
-#pragma unroll
-    for (int r = 0; r < NS; ++r) diag_ok = diag_ok && (fabs(a[r][r]) > 0.0);
-    if (!diag_ok) {
-      bool singular = false;
-#pragma unroll
-      for (int r = 0; r < NS; ++r) {
-        double mx = 0.0;
-#pragma unroll
-        for (int q = 0; q < NS; ++q)
-          if (fabs(a[r][q]) > mx) mx = fabs(a[r][q]);
-        singular = singular || !(mx > 0.0);
+    const double t = lt + (((ns[0] + ns[1]) + (ns[2] + ns[3])) + (ns[4] + ns[5]));
+    if (!(fabs(t) < 1.0e300)) {
+      double n2[NS], p2[NS];
+      for (int s = 0; s < NS; ++s) {
+        n2[s] = ns[s];
+        p2[s] = pw[s];
       }
-      if (singular) atomicOr(st, GITM_ST_LU_SINGULAR);
+      if (friction_singular(dt, n2, p2)) atomicOr(st, GITM_ST_LU_SINGULAR);
     }
   }
+#pragma unroll
+  for (int e = 0; e < NS; ++e) pw[e] = (dt * c_k.kpair[e]) * pw[e];
+  double d[NS], w[NS][NS];  // the diagonal; W below it
+#pragma unroll
+  for (int r = 0; r < NS; ++r) d[r] = mn[r];
+#pragma unroll
+  for (int r = 1; r < NS; ++r)
+#pragma unroll
+    for (int q = 0; q < r; ++q) {
+      w[r][q] = (ns[r] * ns[q]) * pw[exp_index(r, q)];
+      d[r] += w[r][q];
+      d[q] += w[r][q];
+    }
+#pragma unroll
+  for (int r = 0; r < NS; ++r) wv[r] *= mn[r];
 #pragma unroll
   for (int p = 0; p < NS; ++p) {
-    const double ip = 1.0 / a[p][p];
-    a[p][p] = ip;
+    d[p] = rcp_nr(d[p]);
 #pragma unroll
     for (int r = p + 1; r < NS; ++r) {
-      const double l = a[r][p] * ip;
+      const double l = w[r][p] * d[p];
 #pragma unroll
-      for (int q = p + 1; q < NS; ++q) a[r][q] -= l * a[p][q];
-      wv[r] -= l * wv[p];
+      for (int q = p + 1; q < r; ++q) w[r][q] = fma(l, w[q][p], w[r][q]);
+      d[r] = fma(-l, w[r][p], d[r]);
+      wv[r] = fma(l, wv[p], wv[r]);
     }
   }
 #pragma unroll
   for (int r = NS - 1; r >= 0; --r) {
     double sum = wv[r];
 #pragma unroll
-    for (int q = r + 1; q < NS; ++q) sum -= a[r][q] * wv[q];
-    wv[r] = sum * a[r][r];
+    for (int q = r + 1; q < NS; ++q) sum = fma(w[q][r], wv[q], sum);
+    wv[r] = sum * d[r];
   }
-#pragma unroll
-  for (int s = 0; s < NS; ++s) wv[s] = wv[s] + (-eddy * glc[s]);
 }
 
 // GradLogConS at cell i (vertical_solver_rusanov.f90:506-543,
@@ -565,87 +581,99 @@ constexpr double F2 = 0.0416667;  // Factor2, vertical_solver_rusanov.f90:740
 // cell i of the stage state in c, from the limited slopes in c's slope
 // buffer; emit(f, New - state) takes each field's increment.  st (may be
 // null) receives the column's GITM_ST_LU_SINGULAR bit.
+//
+// The stage is bound by the FP64 pipe (two cycles per warp instruction and
+// SM sub-partition), so the increments are formed directly, New - state
+// without the state added and taken off again, and the factors a cell's
+// fields share (dt, the cell width, the dissipation coefficients) are
+// multiplied together once.
 template <class Emit>
 __device__ __forceinline__ void rusanov_cell(ColCtx c, int i, const GitmVertParams& prm, double dt,
                                              double eddy, double ivup, double inv_vert_tau, Emit&& emit,
                                              uint32_t* st = nullptr) {
-  const double dF0 = c.dAF(i), dF1 = c.dAF(i + 1);
   const double idc = c.g(GC_IDC, i);
-  const double fc0 = 0.5 * fmax(c.cm(i - 1), c.cm(i));
-  const double fc1 = 0.5 * fmax(c.cm(i), c.cm(i + 1));
-  // the halves taken once per cell: a product with 0.5 is exact, so
-  // d * (0.5 dF) and x * (0.5 / dAlt_C) round like (0.5 d) dF and (0.5 x) / dAlt_C
-  const double hF0 = 0.5 * dF0, hF1 = 0.5 * dF1, hidc = 0.5 * idc;
-  // calc_rusanov_alts_rusanov (:694-718) at cell i
-  auto sweep = [&](int f, double& grad, double& diff) {
-    const double* v = &c.col[c.xo + f * c.L.G + 1];
-    const double* d = &c.col[c.L.DL + f * (c.L.nAlts + 2)];
+  const double hF0 = 0.5 * c.dAF(i), hF1 = 0.5 * c.dAF(i + 1), hidc = 0.5 * idc;
+  const double hdt = dt * hidc;
+  const double cmi = c.cm(i);
+  const double b0 = hdt * fmax(c.cm(i - 1), cmi);  // dt fc idc of the two faces
+  const double b1 = hdt * fmax(cmi, c.cm(i + 1));
+  // calc_rusanov_alts_rusanov (:694-718) at cell i: grad = ss hidc, dt diff = dd
+  auto sweep = [&](int f, double& ss, double& dd) {
+    const double* v = &c.col[c.xo + f * c.L.P + 1];
+    const double* d = &c.col[c.L.DL + f * c.L.PD];
     const double L0 = fma(d[i - 1], hF0, v[i - 1]);
     const double R0 = fma(-d[i], hF0, v[i]);
     const double L1 = fma(d[i], hF1, v[i]);
     const double R1 = fma(-d[i + 1], hF1, v[i + 1]);
-    grad = (L1 + R1 - L0 - R0) * hidc;
-    diff = (fc1 * (R1 - L1) - fc0 * (R0 - L0)) * idc;
+    ss = L1 + R1 - L0 - R0;
+    dd = fma(b1, R1 - L1, -(b0 * (R0 - L0)));
   };
   const double invr = c.g(GC_INVR, i), rr = c.g(GC_R, i), grav = c.g(GC_GRAV, i);
   const double T = c.x(F_T, i), VE = c.x(F_VE, i), VN = c.x(F_VN, i), VU = c.x(F_VU, i);
-  double gT, dT;
-  sweep(F_T, gT, dT);
+  double gT;
   {
-    double gE, dE, gN, dN, gU, dU;
-    sweep(F_VE, gE, dE);
-    sweep(F_VN, gN, dN);
-    sweep(F_VU, gU, dU);
+    double sT, dT, sE, dE, sN, dN, sU, dU;
+    sweep(F_T, sT, dT);
+    gT = sT * hidc;
+    sweep(F_VE, sE, dE);
+    sweep(F_VN, sN, dN);
+    sweep(F_VU, sU, dU);
     // :660-680
-    emit(F_VE, (VE - dt * VU * gE + dt * dE) - VE);
-    emit(F_VN, (VN - dt * VU * gN + dt * dN) - VN);
-    const double divv = gU + 2 * VU * invr;
-    emit(F_T, (T - dt * (VU * gT + (c.gm(i) - 1.0) * (T * divv)) + dt * dT) - T);
+    const double adv = hdt * VU;
+    emit(F_VE, fma(-adv, sE, dE));
+    emit(F_VN, fma(-adv, sN, dN));
+    const double divv = fma(sU, hidc, 2 * VU * invr);
+    emit(F_T, fma(-dt, fma(VU, gT, (c.gm(i) - 1.0) * (T * divv)), dT));
   }
   // ions 1..nIonsAdvect (:557-568)
+  const double advi = hdt * ivup;
 #pragma unroll
   for (int s = 0; s < NADV; ++s) {
-    double gI, dI;
-    sweep(F_I + s, gI, dI);
-    const double I = c.x(F_I + s, i);
-    emit(F_I + s, (I - dt * (ivup * gI) + dt * dI) - I);
+    double sI, dI;
+    sweep(F_I + s, sI, dI);
+    emit(F_I + s, fma(-advi, sI, dI));
   }
   // species continuity and momentum (:548-617)
   const double itau = prm.use_damping ? 1.0 / (15 - (1 - exp(-1.0 * c.g(GC_ALT, i) / 1000.0 / 40.0)) * 5.0)
                                       : inv_vert_tau;
-  const double hz = (VN * VN + VE * VE) * invr;
-  const double cor = prm.use_coriolis ? dt * (c.sc(SC_CENT) * rr + c.sc(SC_CORI) * VE) : 0.0;
+  const double keep = 1.0 - itau;
+  // what every species' wind takes: dt (horizontal curvature + gravity) and Coriolis
+  double common = dt * fma(VN * VN + VE * VE, invr, grav);
+  if (prm.use_coriolis) common = fma(dt, c.sc(SC_CENT) * rr + c.sc(SC_CORI) * VE, common);
   double wv[NS];
   double sumrho = 0.0;
 #pragma unroll
   for (int s = 0; s < NS; ++s) {
-    double gL, dL, gW, dW;
-    sweep(F_LNS + s, gL, dL);
-    sweep(F_W + s, gW, dW);
+    double sL, dL, sW, dW;
+    sweep(F_LNS + s, sL, dL);
+    sweep(F_W + s, sW, dW);
     const double Ls = c.x(F_LNS + s, i), Ws = c.x(F_W + s, i);
-    const double divw = gW + 2 * Ws * invr;
-    const double nl = Ls - dt * (divw + Ws * gL) + dt * dL;
-    emit(F_LNS + s, nl - Ls);
-    sumrho = sumrho + c_k.mass[s] * exp(nl);
-    const double km = c_k.k_over_m[s];
-    double w = Ws - dt * (Ws * gW - hz + T * gL * km + gT * km - grav) + dt * dW - Ws * itau;
-    w = w + cor;
-    w = w - dt * (prm.thermal_diff_coef[s] * km) * gT;
-    wv[s] = w;
+    const double gL = sL * hidc, gW = sW * hidc;
+    const double kl = fma(-dt, fma(Ws, gL, fma(2 * Ws, invr, gW)), dL);
+    emit(F_LNS + s, kl);
+    sumrho = fma(c_k.mass[s], exp(Ls + kl), sumrho);
+    // the pressure gradient with the thermal diffusion's share of grad T
+    const double pg = fma(T, gL, gT * (1.0 + prm.thermal_diff_coef[s]));
+    wv[s] = fma(-dt, fma(c_k.k_over_m[s], pg, Ws * gW), fma(Ws, keep, common) + dW);
   }
   const double LR = c.x(F_LRHO, i);
   emit(F_LRHO, log(sumrho) - LR);
   // NS = exp(LogNS), 1 / Rho (:466-467)
-  double ns[NS];
+  double ns[NS], mn[NS];
 #pragma unroll
-  for (int s = 0; s < NS; ++s) ns[s] = exp(c.x(F_LNS + s, i));
-  const double ir = exp(-LR);
+  for (int s = 0; s < NS; ++s) {
+    ns[s] = exp(c.x(F_LNS + s, i));
+    mn[s] = c_k.mass[s] * ns[s];
+  }
   // calc_neutral_friction (calc_neutral_friction.f90:47-106)
   if (prm.use_neutral_friction) {
-    // GradLogConS (:506-543), LogConS = log(m_s) + LogNS - LogRho
-    double glc[NS];
-    grad_log_cons(c, i, glc);
-    friction_solve(dt, ns, T, eddy, glc, wv, st);
+    friction_solve(dt, ns, mn, T, wv, st);
+    if (eddy != 0.0) {  // the coefficient is zero above the turbopause: most cells
+      double glc[NS];  // GradLogConS (:506-543), LogConS = log(m_s) + LogNS - LogRho
+      grad_log_cons(c, i, glc);
+#pragma unroll
+      for (int s = 0; s < NS; ++s) wv[s] = fma(-eddy, glc[s], wv[s]);
+    }
   }
   // clamp and bulk vertical wind (:643-658)
   double vu = 0.0;
@@ -654,9 +682,9 @@ __device__ __forceinline__ void rusanov_cell(ColCtx c, int i, const GitmVertPara
     double w = fmax(-prm.max_vertical_velocity, wv[s]);
     w = fmin(prm.max_vertical_velocity, w);
     emit(F_W + s, w - c.x(F_W + s, i));
-    vu = vu + w * (c_k.mass[s] * ns[s] * ir);
+    vu = fma(w, mn[s], vu);
   }
-  emit(F_VU, vu - VU);
+  emit(F_VU, fma(vu, exp(-LR), -VU));
 }
 
 // Limited slopes of the 18 swept fields at cell i: the 4th-order form on
