@@ -7,7 +7,8 @@
 Every translation unit is compiled to an object in gitm_b200/_build (in
 parallel), then the objects are linked into the shared library.  The step
 kernel is compiled once per entry of GV_STEP_INSTANCES (csrc/vert_instances.h),
-each in a unit of its own (csrc/vert_instance.cu with that entry's -D values).
+each in a unit of its own (csrc/vert_instance.cu with that entry's -D values),
+and so is the tile kernel per entry of GV_TILE_INSTANCES (csrc/vert_tile.cu).
 """
 from __future__ import annotations
 
@@ -23,7 +24,7 @@ BUILD = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libgitmvert.so")
 SOURCES = ["gitm_vert.cu", "vert_adjoint.cu", "hz_kernel.cu"]
 DEPS = ["gitm_vert.cu", "vert_adjoint.cu", "hz_kernel.cu", "vert_instance.cu", "vert_instances.h", "vert_kernel.cuh",
-        "vert_ausm.cuh", "vert_adjoint.cuh", "vert_common.cuh", "vert_hz.cuh", "vert_math.cuh"]
+        "vert_ausm.cuh", "vert_adjoint.cuh", "vert_common.cuh", "vert_hz.cuh", "vert_math.cuh", "vert_tile.cu", "vert_tile.cuh"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -55,6 +56,17 @@ def instances() -> list[tuple[str, list[str]]]:
     return out
 
 
+def tile_instances() -> list[tuple[str, list[str]]]:
+    """(id, -D flags) of every GV_TILE_INSTANCES entry."""
+    text = open(os.path.join(CSRC, "vert_instances.h")).read()
+    body = text[text.index("#define GV_TILE_INSTANCES(T)"):].split("\n\n", 1)[0]
+    out = [(gid, [f"-DGV_ID={gid}", f"-DGV_SAVE={save}", f"-DGV_NA={na}"])
+           for gid, save, na in re.findall(r"T\((\w+),\s*(true|false),\s*(\d+)\)", body)]
+    if not out:
+        raise RuntimeError("no tile-kernel instances found in vert_instances.h")
+    return out
+
+
 def stale() -> bool:
     if not os.path.exists(LIB):
         return True
@@ -76,6 +88,8 @@ def build(force: bool = False, verbose: bool = False) -> str:
     jobs.append((os.path.join(CSRC, "vert_adjoint.cu"), ["-DGV_ADJ_NA=50"], os.path.join(BUILD, "vert_adjoint_n50.o")))
     jobs += [(os.path.join(CSRC, "vert_instance.cu"), flags, os.path.join(BUILD, f"step_{gid}.o"))
              for gid, flags in instances()]
+    jobs += [(os.path.join(CSRC, "vert_tile.cu"), flags, os.path.join(BUILD, f"step_{gid}.o"))
+             for gid, flags in tile_instances()]
 
     def compile_one(job):
         src, flags, obj = job

@@ -19,6 +19,7 @@
 
 #include "vert_common.cuh"
 #include "vert_kernel.cuh"
+#include "vert_tile.cuh"
 #include "vert_adjoint.cuh"
 #include "vert_instances.h"
 #include "vert_hz.cuh"
@@ -238,16 +239,17 @@ static void grid_coefs(int nA, const double* alt, const double* grav, const doub
 // Launch shapes built: threads per CTA -> CTAs per SM the registers allow and
 // where the RK accumulator lives.  The small CTAs keep it in a per-CTA slot
 // of global scratch (L2-resident under their persistent grid) so that two or
-// three CTAs share an SM and overlap each other's barrier phases.
-// The 512-thread shape also keeps Orig in its scratch slot (orig_global):
-// 8 columns of 50 altitudes then fit the shared memory of an SM, 16 warps at
-// 128 registers.  The AUSM solver's 384-thread shape does the same (6
-// columns of its larger slot instead of 4).  solver -1: any solver.
-struct Shape { int threads, solver, min_blocks; bool acc_global, orig_global; };
-static const Shape kShapes[] = {{128, -1, 3, true, false}, {160, -1, 2, true, false}, {192, -1, 2, true, false},
-                                {256, -1, 1, false, false}, {320, -1, 1, false, false},
-                                {384, GITM_SOLVER_AUSM, 1, true, true}, {384, -1, 1, false, false},
-                                {512, -1, 1, true, true}};
+// three CTAs share an SM and overlap each other's barrier phases.  The AUSM
+// solver's 384-thread shape also keeps Orig there (orig_global: 6 columns of
+// its larger slot instead of 4).  The Rusanov solver's 512-thread shape is
+// the tile kernel (vert_tile.cuh), which holds both in tensor memory.
+// solver -1: any solver.
+struct Shape { int threads, solver, min_blocks; bool acc_global, orig_global, tile; };
+static const Shape kShapes[] = {{128, -1, 3, true, false, false}, {160, -1, 2, true, false, false},
+                                {192, -1, 2, true, false, false}, {256, -1, 1, false, false, false},
+                                {320, -1, 1, false, false, false},
+                                {384, GITM_SOLVER_AUSM, 1, true, true, false}, {384, -1, 1, false, false, false},
+                                {512, GITM_SOLVER_RUSANOV, 1, false, false, true}};
 static const int kThreadChoices[] = {128, 160, 192, 256, 320, 384, 512};
 
 static const Shape* shape_of(int threads, int solver) {
@@ -266,6 +268,17 @@ static bool orig_global(int threads, int solver) {
   return s && s->orig_global;
 }
 
+static bool tile_shape(int threads, int solver) {
+  const Shape* s = shape_of(threads, solver);
+  return s && s->tile;
+}
+
+// Dynamic shared memory of a CTA of that shape holding nc columns.
+static size_t shape_smem(int threads, int solver, int nAlts, int nc) {
+  return tile_shape(threads, solver) ? tile_smem_bytes(nAlts, nc)
+                                     : smem_bytes(nAlts, nc, solver, orig_global(threads, solver));
+}
+
 // The step kernels, each compiled in its own translation unit
 // (vert_instance.cu, one per GV_STEP_INSTANCES entry).
 struct StepInstance {
@@ -280,6 +293,10 @@ static const StepInstance kInstances[] = {
   {IO, NT, SOLVER, SAVE, NA, step_kernel_##id, step_consts_##id},
     GV_STEP_INSTANCES(GV_TABLE_ENTRY)
 #undef GV_TABLE_ENTRY
+#define GV_TABLE_TILE(id, SAVE, NA) \
+  {0, TILE_THREADS, GITM_SOLVER_RUSANOV, SAVE, NA, step_kernel_##id, step_consts_##id},
+    GV_TILE_INSTANCES(GV_TABLE_TILE)
+#undef GV_TABLE_TILE
 };
 
 // The step kernel for an array form (0 GITM arrays, 1 ModVertical), solver
@@ -417,9 +434,9 @@ int gitm_vert_set_params(GitmVertCtx* ctx, const GitmVertParams* params) {
 // Columns per CTA for a member of nAlts under cfg.
 static int cols_per_cta(const GitmVertCtx* ctx, const GitmLaunchConfig& cfg, int nA, int solver) {
   int nc = cfg.cols_per_cta > 0 ? cfg.cols_per_cta : cfg.threads / nA;
-  nc = std::min(nc, cfg.threads / 32);  // one BC warp per column
+  if (!tile_shape(cfg.threads, solver)) nc = std::min(nc, cfg.threads / 32);  // one BC warp per column
   nc = std::min(nc, cfg.threads / nA);  // every interior cell has a thread
-  while (nc > 1 && smem_bytes(nA, nc, solver, orig_global(cfg.threads, solver)) > ctx->max_smem) --nc;
+  while (nc > 1 && shape_smem(cfg.threads, solver, nA, nc) > ctx->max_smem) --nc;
   return std::max(nc, 1);
 }
 
@@ -434,10 +451,11 @@ static int build_tiles(GitmVertPlan* P) {
   for (int m = 0; m < P->n_members; ++m) {
     const GitmColumnBatch& b = P->host_members[m];
     const int nc = cols_per_cta(ctx, P->cfg, b.n_alts, P->solver);
-    if (nc * b.n_alts > P->cfg.threads || smem_bytes(b.n_alts, nc, P->solver, og) > ctx->max_smem)
+    const size_t need = shape_smem(P->cfg.threads, P->solver, b.n_alts, nc);
+    if (nc * b.n_alts > P->cfg.threads || need > ctx->max_smem)
       return set_err(ctx, GITM_ERR_ARG, "nAlts %d does not fit a CTA of %d threads", b.n_alts,
                      P->cfg.threads);
-    P->smem = std::max(P->smem, smem_bytes(b.n_alts, nc, P->solver, og));
+    P->smem = std::max(P->smem, need);
     if (og) orig_per_cta = std::max(orig_per_cta, size_t(nc) * orig_doubles(b.n_alts));
     for (int64_t c0 = 0; c0 < b.n_cols; c0 += nc) {
       Tile t;
@@ -459,7 +477,7 @@ static int build_tiles(GitmVertPlan* P) {
   const int T = P->cfg.threads;
   int grid = int(P->tiles.size());
   int per_sm = P->cfg.ctas_per_sm;
-  if (acc_global(T, P->solver) && per_sm <= 0) {
+  if ((acc_global(T, P->solver) || tile_shape(T, P->solver)) && per_sm <= 0) {
     const void* fn = kernel_for(P->io, P->solver, T, plan_nalts(P));
     CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, T, P->smem));
     per_sm = std::max(per_sm, 1);

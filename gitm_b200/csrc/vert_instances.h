@@ -15,8 +15,10 @@
 // members of exactly that nAlts (GITM's default 50), whose shared-memory
 // offsets and loop bounds are compile-time constants; the host launches it
 // when every member of a plan has that nAlts.  OG: Orig in global scratch
-// (the 512-thread shape: 8 columns of 50 altitudes, 16 warps per SM at 128
-// registers).
+// (the AUSM solver's 384-thread shape).
+//
+// GV_TILE_INSTANCES lists the 512-thread shape of the Rusanov solver on GITM
+// arrays, a kernel of its own (vert_tile.cuh): T(id, SAVE, NA).
 #pragma once
 
 #include "vert_common.cuh"
@@ -46,9 +48,11 @@
   X(ausm0_t128_n50, 0, 128, 2, true, 1, false, 50, false)     \
   X(ausm0_t256_n50, 0, 256, 1, false, 1, false, 50, false)    \
   X(rus0_t128_save_n50, 0, 128, 3, true, 0, true, 50, false)  \
-  X(rus0_t512_og, 0, 512, 1, true, 0, false, 0, true)         \
-  X(rus0_t512_og_n50, 0, 512, 1, true, 0, false, 50, true)    \
   X(ausm0_t384_og_n50, 0, 384, 1, true, 1, false, 50, true)
+
+#define GV_TILE_INSTANCES(T)     \
+  T(tile, false, 0)              \
+  T(tile_n50, false, 50)
 
 namespace gv {
 #define GV_DECLARE_INSTANCE(id, IO, NT, MINB, ACC, SOLVER, SAVE, NA, OG) \
@@ -56,4 +60,9 @@ namespace gv {
   cudaError_t step_consts_##id(const Consts& k);
 GV_STEP_INSTANCES(GV_DECLARE_INSTANCE)
 #undef GV_DECLARE_INSTANCE
+#define GV_DECLARE_TILE(id, SAVE, NA) \
+  const void* step_kernel_##id();     \
+  cudaError_t step_consts_##id(const Consts& k);
+GV_TILE_INSTANCES(GV_DECLARE_TILE)
+#undef GV_DECLARE_TILE
 }  // namespace gv

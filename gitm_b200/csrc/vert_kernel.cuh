@@ -115,13 +115,18 @@ __device__ __forceinline__ bool photochemical(int s) { return s == 3 || s == 4; 
 // ModLimiter.f90:16-36, without branches: on same-sign slopes the smallest
 // magnitude of beta u, beta d and (u + d) / 2 carries the common sign (the
 // reference's min of the three when both are positive and max when both are
-// negative, the same values since negation is exact); 0 otherwise.  Lanes
-// whose cells take different cases do not split the warp.
+// negative, the same values since negation is exact and rounding monotonic:
+// min(beta |u|, beta |d|) = beta min(|u|, |d|)); 0 otherwise.  Selects on
+// plain comparisons and the sign bits: fmin and the four comparisons with
+// zero took about twice the instructions.
 __device__ __forceinline__ double limiter_mc(double u, double d, double beta) {
-  const double m = fmin(fmin(fabs(beta * u), fabs(beta * d)), fabs((u + d) * 0.5));
-  const bool pos = (u > 0.0) && (d > 0.0);
-  const bool neg = !(u > 0.0) && (d < 0.0);
-  return pos ? m : (neg ? -m : 0.0);
+  const double au = fabs(u), ad = fabs(d);
+  const double t = beta * (au < ad ? au : ad);
+  const double s = (u + d) * 0.5, as = fabs(s);
+  const double m = t < as ? t : as;
+  const bool same = (__double2hiint(u) ^ __double2hiint(d)) >= 0;  // a zero among them makes m zero
+  const int hi = __double2hiint(m) | (__double2hiint(u) & int(0x80000000u));
+  return same ? __hiloint2double(hi, __double2loint(m)) : 0.0;
 }
 
 struct ColCtx {
@@ -498,22 +503,30 @@ static __device__ __noinline__ bool friction_singular(double dt, const double* n
 // solver at 2.5 degrees, 4 steps, 11.45 -> 10.60 ms).
 // mn[s] = M_s n_s.  A non-finite density or temperature takes the reference's
 // row test, which sets GITM_ST_LU_SINGULAR in *st (when st is given); the
-// solve goes on, its results non-finite.
+// solve goes on, its results non-finite.  WARP: whole warps call it, and no
+// branch splits them (the caller's next instruction needs the warp converged).
+template <bool WARP = false>
 __device__ __forceinline__ void friction_solve(double dt, const double (&ns)[NS], const double (&mn)[NS], double T,
                                                double (&wv)[NS], uint32_t* st = nullptr) {
-  const double lt = log(T);
-  double pw[NS];
+  const double T1[1] = {T};
+  double l1[1];
+  log_n<1, WARP>(T1, l1);
+  const double lt = l1[0];
+  double pw[NS], le[NS];
 #pragma unroll
-  for (int e = 0; e < NS; ++e) pw[e] = exp(c_k.one_minus_e[e] * lt);
+  for (int e = 0; e < NS; ++e) le[e] = c_k.one_minus_e[e] * lt;
+  exp_n<NS, WARP>(le, pw);
   if (st) {
     const double t = lt + (((ns[0] + ns[1]) + (ns[2] + ns[3])) + (ns[4] + ns[5]));
-    if (!(fabs(t) < 1.0e300)) {
+    const bool odd = !(fabs(t) < 1.0e300);
+    if (WARP ? __any_sync(0xffffffffu, odd) : odd) {
       double n2[NS], p2[NS];
       for (int s = 0; s < NS; ++s) {
         n2[s] = ns[s];
         p2[s] = pw[s];
       }
-      if (friction_singular(dt, n2, p2)) atomicOr(st, GITM_ST_LU_SINGULAR);
+      if (friction_singular(dt, n2, p2) && odd) atomicOr(st, GITM_ST_LU_SINGULAR);
+      if (WARP) __syncwarp();
     }
   }
 #pragma unroll
@@ -586,8 +599,8 @@ constexpr double F2 = 0.0416667;  // Factor2, vertical_solver_rusanov.f90:740
 // SM sub-partition), so the increments are formed directly, New - state
 // without the state added and taken off again, and the factors a cell's
 // fields share (dt, the cell width, the dissipation coefficients) are
-// multiplied together once.
-template <class Emit>
+// multiplied together once.  WARP as in friction_solve.
+template <bool WARP = false, class Emit>
 __device__ __forceinline__ void rusanov_cell(ColCtx c, int i, const GitmVertParams& prm, double dt,
                                              double eddy, double ivup, double inv_vert_tau, Emit&& emit,
                                              uint32_t* st = nullptr) {
@@ -640,8 +653,7 @@ __device__ __forceinline__ void rusanov_cell(ColCtx c, int i, const GitmVertPara
   // what every species' wind takes: dt (horizontal curvature + gravity) and Coriolis
   double common = dt * fma(VN * VN + VE * VE, invr, grav);
   if (prm.use_coriolis) common = fma(dt, c.sc(SC_CENT) * rr + c.sc(SC_CORI) * VE, common);
-  double wv[NS];
-  double sumrho = 0.0;
+  double wv[NS], nl[NS];
 #pragma unroll
   for (int s = 0; s < NS; ++s) {
     double sL, dL, sW, dW;
@@ -651,24 +663,40 @@ __device__ __forceinline__ void rusanov_cell(ColCtx c, int i, const GitmVertPara
     const double gL = sL * hidc, gW = sW * hidc;
     const double kl = fma(-dt, fma(Ws, gL, fma(2 * Ws, invr, gW)), dL);
     emit(F_LNS + s, kl);
-    sumrho = fma(c_k.mass[s], exp(Ls + kl), sumrho);
+    nl[s] = Ls + kl;
     // the pressure gradient with the thermal diffusion's share of grad T
     const double pg = fma(T, gL, gT * (1.0 + prm.thermal_diff_coef[s]));
     wv[s] = fma(-dt, fma(c_k.k_over_m[s], pg, Ws * gW), fma(Ws, keep, common) + dW);
   }
   const double LR = c.x(F_LRHO, i);
-  emit(F_LRHO, log(sumrho) - LR);
-  // NS = exp(LogNS), 1 / Rho (:466-467)
   double ns[NS], mn[NS];
+  exp_n<NS, WARP>(nl, ns);
+  {
+    double rho[1] = {0.0}, lr[1];
 #pragma unroll
-  for (int s = 0; s < NS; ++s) {
-    ns[s] = exp(c.x(F_LNS + s, i));
-    mn[s] = c_k.mass[s] * ns[s];
+    for (int s = 0; s < NS; ++s) rho[0] = fma(c_k.mass[s], ns[s], rho[0]);
+    log_n<1, WARP>(rho, lr);
+    emit(F_LRHO, lr[0] - LR);
+  }
+  // NS = exp(LogNS), 1 / Rho (:466-467)
+  double ir;
+  {
+    double l7[NS + 1], e7[NS + 1];
+#pragma unroll
+    for (int s = 0; s < NS; ++s) l7[s] = c.x(F_LNS + s, i);
+    l7[NS] = -LR;
+    exp_n<NS + 1, WARP>(l7, e7);
+#pragma unroll
+    for (int s = 0; s < NS; ++s) {
+      ns[s] = e7[s];
+      mn[s] = c_k.mass[s] * ns[s];
+    }
+    ir = e7[NS];
   }
   // calc_neutral_friction (calc_neutral_friction.f90:47-106)
   if (prm.use_neutral_friction) {
-    friction_solve(dt, ns, mn, T, wv, st);
-    if (eddy != 0.0) {  // the coefficient is zero above the turbopause: most cells
+    friction_solve<WARP>(dt, ns, mn, T, wv, st);
+    if (WARP ? __any_sync(0xffffffffu, eddy != 0.0) : eddy != 0.0) {  // the coefficient is zero above the turbopause: most cells
       double glc[NS];  // GradLogConS (:506-543), LogConS = log(m_s) + LogNS - LogRho
       grad_log_cons(c, i, glc);
 #pragma unroll
@@ -679,12 +707,12 @@ __device__ __forceinline__ void rusanov_cell(ColCtx c, int i, const GitmVertPara
   double vu = 0.0;
 #pragma unroll
   for (int s = 0; s < NS; ++s) {
-    double w = fmax(-prm.max_vertical_velocity, wv[s]);
-    w = fmin(prm.max_vertical_velocity, w);
+    double w = (wv[s] > -prm.max_vertical_velocity) ? wv[s] : -prm.max_vertical_velocity;
+    w = (w < prm.max_vertical_velocity) ? w : prm.max_vertical_velocity;
     emit(F_W + s, w - c.x(F_W + s, i));
     vu = fma(w, mn[s], vu);
   }
-  emit(F_VU, fma(vu, exp(-LR), -VU));
+  emit(F_VU, fma(vu, ir, -VU));
 }
 
 // Limited slopes of the 18 swept fields at cell i: the 4th-order form on
@@ -978,6 +1006,7 @@ __global__ void __launch_bounds__(NT, MINB) vert_step_kernel(const KParams kp) {
     double eddy = 0.0, ivup = 0.0;
     double accr[ACC_GLOBAL ? 1 : NF];
 
+#pragma unroll 1
     for (int step = 0; step < kp.n_steps; ++step) {
       if (item) {
         if (IO == 0) {
@@ -1015,6 +1044,7 @@ __global__ void __launch_bounds__(NT, MINB) vert_step_kernel(const KParams kp) {
         }
       }
 
+#pragma unroll 1
       for (int k = 0; k < 4; ++k) {
         // -------------------------------------------------- phase A
         if constexpr (SOLVER == GITM_SOLVER_AUSM) {

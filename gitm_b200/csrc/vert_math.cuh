@@ -1,26 +1,40 @@
-// vert_math.cuh -- the FP64 reciprocal of the friction solves, as plain
-// multiply-adds.
+// vert_math.cuh -- FP64 exp, log and reciprocal for the stage kernels.
 //
-// CUDA's division ends in a range test with a slow path behind a branch; the
-// six pivots of a friction solve are a serial chain, and each branch ends the
-// block the compiler can schedule over.  rcp_nr refines PTX's documented
-// rcp.approx.ftz.f64 (relative error 2^-23) with two Newton-Raphson steps:
-// four FP64 instructions.  The header also compiles as plain C++, for
-// tests/test_math.py.
+// What bounds a stage is the number of instructions its warps issue and the
+// latency of their FP64 chains.  CUDA's exp is 15 FP64 instructions among 49
+// (log: 30 of 81; their range tests, special cases and literal constants are
+// the rest), and ends in a branch, so the calls of a loop over species run
+// one after the other.  The batches here run N arguments side by side with
+// one range test for all: 18 instructions per exp (15 FP64), 32 per log (23),
+// 5 per reciprocal.
+//
+// Written from the mathematics.  The range reduction is Cody and Waite's
+// (Software Manual for the Elementary Functions, 1980: ln 2 in two parts),
+// the polynomials are Chebyshev interpolants of (e^r - 1 - r) / r^2 on
+// |r| <= 0.347 (truncation 1.7e-17 relative) and of the atanh series on the
+// mantissas of [sqrt(1/2), sqrt(2)) (4.7e-18), the reciprocal refines PTX's
+// documented rcp.approx.ftz.f64 with Newton-Raphson steps.  Error against
+// the exact value: at most 0.94 ulp (exp), 0.96 ulp (log), 1 ulp
+// (reciprocal); tests/test_math.py, which compiles the header as plain C++.
 #pragma once
 
 #include <cstdint>
 #ifdef __CUDACC__
 #define GV_MATH __device__ __forceinline__
+#define GV_UNROLL _Pragma("unroll")
 #else
 #include <cmath>
 #include <cstring>
 #define GV_MATH inline
+#define GV_UNROLL
 #endif
 
 namespace gv {
 
 #ifdef __CUDACC__
+GV_MATH int m_hi(double x) { return __double2hiint(x); }
+GV_MATH int m_lo(double x) { return __double2loint(x); }
+GV_MATH double m_make(int hi, int lo) { return __hiloint2double(hi, lo); }
 GV_MATH double m_fma(double a, double b, double c) { return fma(a, b, c); }
 GV_MATH double rcp_seed(double a) {
   double r;
@@ -28,24 +42,171 @@ GV_MATH double rcp_seed(double a) {
   return r;
 }
 #else
-GV_MATH double m_fma(double a, double b, double c) { return std::fma(a, b, c); }
-// a seed of the documented accuracy where there is no GPU: 22 bits of 1 / a
-GV_MATH double rcp_seed(double a) {
-  double r = 1.0 / a;
+GV_MATH int m_hi(double x) {
   uint64_t u;
-  std::memcpy(&u, &r, 8);
-  u &= 0xffffffffc0000000ull;
-  std::memcpy(&r, &u, 8);
-  return r;
+  std::memcpy(&u, &x, 8);
+  return int(uint32_t(u >> 32));
+}
+GV_MATH int m_lo(double x) {
+  uint64_t u;
+  std::memcpy(&u, &x, 8);
+  return int(uint32_t(u));
+}
+GV_MATH double m_make(int hi, int lo) {
+  const uint64_t u = (uint64_t(uint32_t(hi)) << 32) | uint32_t(lo);
+  double x;
+  std::memcpy(&x, &u, 8);
+  return x;
+}
+GV_MATH double m_fma(double a, double b, double c) { return std::fma(a, b, c); }
+// a seed of the documented accuracy (23 bits) where there is no GPU
+GV_MATH double rcp_seed(double a) {
+  const double r = 1.0 / a;
+  return m_make(m_hi(r), m_lo(r) & int(0xc0000000u));
 }
 #endif
 
-// 1 / a.  Relative error at most 1 ulp for |a| in [2^-1020, 2^1020]; a zero,
-// subnormal, infinite or NaN argument gives a result that is not finite.
+// The constants are read from constant memory, where an FP64 instruction
+// takes them as an operand: as literals each costs two moves and a register
+// pair.
+#ifdef __CUDACC__
+static __constant__ double
+#else
+static const double
+#endif
+    m_k[] = {
+        1.4426950408889634,      // 0: log2 e
+        0.6931471805582987,      // 1: ln 2 to 38 fraction bits: n times it is exact
+        1.6465949582897082e-12,  // 2: the rest of ln 2
+        6755399441055744.0,      // 3: 1.5 * 2^52: adding it rounds to an integer
+        // 4..13: (e^r - 1 - r) / r^2, highest power first
+        2.5100494788905042e-08, 2.76202305675069e-07, 2.7557268229963227e-06, 2.4801520996825697e-05,
+        0.00019841269863201828, 0.0013888888917406447, 0.008333333333330032, 0.04166666666662374,
+        0.16666666666666669, 0.5000000000000001,
+        // 14..20: (2 atanh(s) - 2 s) / s^3 in s^2, highest power first
+        0.1461916477718642, 0.1533150172120742, 0.18182895746801428, 0.22222211043822487,
+        0.28571428626533335, 0.3999999999989827, 0.666666666666667};
+
+// 1 / a.  Relative error below 1 ulp for |a| in [2^-1020, 2^1020]; outside
+// (0, infinities, NaN, subnormals) the result is not finite or NaN.
 GV_MATH double rcp_nr(double a) {
   double r = rcp_seed(a);
   r = m_fma(r, m_fma(-a, r, 1.0), r);
   return m_fma(r, m_fma(-a, r, 1.0), r);
+}
+
+// CUDA's own functions, out of line: the batches below take them for the
+// arguments outside their fast range.
+#ifdef __CUDACC__
+static __device__ __noinline__ double exp_any(double x) { return exp(x); }
+static __device__ __noinline__ double log_any(double x) { return log(x); }
+#else
+inline double exp_any(double x) { return std::exp(x); }
+inline double log_any(double x) { return std::log(x); }
+#endif
+
+// Whether the far branch is taken.  WARP: by whole warps (the caller's warp
+// is converged and has to stay so), else lane by lane.
+template <bool WARP>
+GV_MATH bool m_any(bool far) {
+#ifdef __CUDACC__
+  if (WARP) return __any_sync(0xffffffffu, far);
+#endif
+  return far;
+}
+
+// The batches run step by step over their N arguments: in source order N
+// independent chains side by side, which is also how they are issued (a loop
+// over whole calls came out one call after the other).
+
+// y = e^x for every x.
+template <int N, bool WARP = false>
+GV_MATH void exp_n(const double (&x)[N], double (&y)[N]) {
+  double r[N], p[N];
+  int n[N], top = 0;
+  GV_UNROLL for (int j = 0; j < N; ++j) {
+    const int ax = m_hi(x[j]) & 0x7fffffff;
+    top = ax > top ? ax : top;
+    p[j] = m_fma(x[j], m_k[0], m_k[3]);
+  }
+  GV_UNROLL for (int j = 0; j < N; ++j) {
+    n[j] = m_lo(p[j]);
+    p[j] = p[j] - m_k[3];
+  }
+  GV_UNROLL for (int j = 0; j < N; ++j) r[j] = m_fma(-p[j], m_k[1], x[j]);
+  GV_UNROLL for (int j = 0; j < N; ++j) r[j] = m_fma(-p[j], m_k[2], r[j]);
+  GV_UNROLL for (int j = 0; j < N; ++j) p[j] = m_fma(m_k[4], r[j], m_k[5]);
+  GV_UNROLL for (int k = 6; k < 14; ++k)
+    GV_UNROLL for (int j = 0; j < N; ++j) p[j] = m_fma(p[j], r[j], m_k[k]);
+  GV_UNROLL for (int j = 0; j < N; ++j) p[j] = m_fma(p[j], r[j], 1.0);
+  GV_UNROLL for (int j = 0; j < N; ++j) p[j] = m_fma(p[j], r[j], 1.0);
+  // times 2^n in the exponent field: a normal number for |x| < 708
+  GV_UNROLL for (int j = 0; j < N; ++j) y[j] = m_make(m_hi(p[j]) + (n[j] << 20), m_lo(p[j]));
+  const bool far = top >= 0x40862000;  // |x| >= 708, infinities, NaN
+  if (m_any<WARP>(far)) {
+    GV_UNROLL for (int j = 0; j < N; ++j) {
+      const double v = exp_any(x[j]);
+      y[j] = far ? v : y[j];
+    }
+  }
+}
+
+// y = log x for every x.
+template <int N, bool WARP = false>
+GV_MATH void log_n(const double (&x)[N], double (&y)[N]) {
+  double f[N], d[N], r[N], s[N], z[N], p[N];
+  int e[N];
+  bool far = false;  // not a normal positive number
+  GV_UNROLL for (int j = 0; j < N; ++j) {
+    // mantissa in [sqrt(1/2), sqrt(2)): offset the exponent field by that of sqrt(1/2)
+    far = far || unsigned(m_hi(x[j])) - 0x00100000u >= 0x7fe00000u;
+    const int hm = m_hi(x[j]) + (0x3ff00000 - 0x3fe6a09e);
+    e[j] = (hm >> 20) - 1023;
+    const double m = m_make((hm & 0x000fffff) + 0x3fe6a09e, m_lo(x[j]));
+    f[j] = m - 1.0;
+    d[j] = m + 1.0;
+  }
+  // s = f / d, the quotient corrected by its residual
+  GV_UNROLL for (int j = 0; j < N; ++j) r[j] = rcp_seed(d[j]);
+  GV_UNROLL for (int j = 0; j < N; ++j) s[j] = m_fma(-d[j], r[j], 1.0);
+  GV_UNROLL for (int j = 0; j < N; ++j) r[j] = m_fma(r[j], s[j], r[j]);
+  GV_UNROLL for (int j = 0; j < N; ++j) s[j] = f[j] * r[j];
+  GV_UNROLL for (int j = 0; j < N; ++j) z[j] = m_fma(-d[j], s[j], f[j]);
+  GV_UNROLL for (int j = 0; j < N; ++j) s[j] = m_fma(z[j], r[j], s[j]);
+  GV_UNROLL for (int j = 0; j < N; ++j) z[j] = s[j] * s[j];
+  GV_UNROLL for (int j = 0; j < N; ++j) p[j] = m_fma(m_k[14], z[j], m_k[15]);
+  GV_UNROLL for (int k = 16; k < 21; ++k)
+    GV_UNROLL for (int j = 0; j < N; ++j) p[j] = m_fma(p[j], z[j], m_k[k]);
+  // log m = 2 s + s z p, with f = 2 s + s f: f - s (f - z p) keeps f's bits
+  GV_UNROLL for (int j = 0; j < N; ++j) p[j] = m_fma(-z[j], p[j], f[j]);
+  GV_UNROLL for (int j = 0; j < N; ++j) p[j] = -s[j] * p[j];
+  GV_UNROLL for (int j = 0; j < N; ++j) {
+    const double ed = m_make(0x43300000, e[j] ^ int(0x80000000u)) - 4503601774854144.0;  // e as a double
+    // e ln2 + f with its rounding error carried (|e ln2| > |f| or e = 0)
+    const double eh = ed * m_k[1];
+    const double b = eh + f[j];
+    y[j] = b + ((f[j] - (b - eh)) + m_fma(ed, m_k[2], p[j]));
+  }
+  if (m_any<WARP>(far)) {
+    GV_UNROLL for (int j = 0; j < N; ++j) {
+      const double v = log_any(x[j]);
+      y[j] = far ? v : y[j];
+    }
+  }
+}
+
+GV_MATH double exp_sl(double x) {
+  const double a[1] = {x};
+  double y[1];
+  exp_n(a, y);
+  return y[0];
+}
+
+GV_MATH double log_sl(double x) {
+  const double a[1] = {x};
+  double y[1];
+  log_n(a, y);
+  return y[0];
 }
 
 }  // namespace gv
