@@ -94,7 +94,6 @@ struct GitmVertPlan {
   Tile* d_save_tiles = nullptr;
   int save_grid = 0;
   size_t save_smem = 0;
-  double* d_save_scratch = nullptr;
 };
 
 static int set_err(GitmVertCtx* ctx, int code, const char* fmt, ...) {
@@ -289,8 +288,8 @@ struct StepInstance {
   cudaError_t (*consts)(const Consts&);
 };
 static const StepInstance kInstances[] = {
-#define GV_TABLE_ENTRY(id, IO, NT, MINB, ACC, SOLVER, SAVE, NA, OG) \
-  {IO, NT, SOLVER, SAVE, NA, step_kernel_##id, step_consts_##id},
+#define GV_TABLE_ENTRY(id, IO, NT, MINB, ACC, SOLVER, NA, OG) \
+  {IO, NT, SOLVER, false, NA, step_kernel_##id, step_consts_##id},
     GV_STEP_INSTANCES(GV_TABLE_ENTRY)
 #undef GV_TABLE_ENTRY
 #define GV_TABLE_TILE(id, SAVE, NA) \
@@ -440,6 +439,19 @@ static int cols_per_cta(const GitmVertCtx* ctx, const GitmLaunchConfig& cfg, int
   return std::max(nc, 1);
 }
 
+// The tile kernel runs one CTA per SM and a tile takes nearly the same time
+// whatever it holds, so where a launch is a few rounds of tiles what counts is
+// the number of rounds: each member's tiles are made as small as the same
+// number of rounds allows, which shares the columns evenly over the SMs (324
+// columns of 50 altitudes: 3 per tile on 108 SMs instead of 10 on 33; 2,592:
+// 9 per tile, two rounds of 144).  Returns the share of a full tile.
+static double tile_share(const GitmVertCtx* ctx, const std::vector<std::pair<int64_t, int>>& cols_and_full) {
+  double load = 0.0;
+  for (const auto& m : cols_and_full) load += double(m.first) / m.second;
+  const double rounds = std::ceil(load / ctx->num_sms);
+  return (rounds >= 1.0 && rounds <= 8.0) ? load / (rounds * ctx->num_sms) : 1.0;
+}
+
 static int build_tiles(GitmVertPlan* P) {
   GitmVertCtx* ctx = P->ctx;
   if (!kernel_for(P->io, P->solver, P->cfg.threads, plan_nalts(P)))
@@ -448,9 +460,17 @@ static int build_tiles(GitmVertPlan* P) {
   P->smem = 0;
   const bool og = orig_global(P->cfg.threads, P->solver);
   size_t orig_per_cta = 0;  // doubles of Orig a CTA's scratch slot holds (orig_global shapes)
+  double share = 1.0;
+  if (tile_shape(P->cfg.threads, P->solver) && P->cfg.cols_per_cta <= 0) {
+    std::vector<std::pair<int64_t, int>> full;
+    for (const GitmColumnBatch& b : P->host_members)
+      full.push_back({b.n_cols, cols_per_cta(ctx, P->cfg, b.n_alts, P->solver)});
+    share = tile_share(ctx, full);
+  }
   for (int m = 0; m < P->n_members; ++m) {
     const GitmColumnBatch& b = P->host_members[m];
-    const int nc = cols_per_cta(ctx, P->cfg, b.n_alts, P->solver);
+    const int most = cols_per_cta(ctx, P->cfg, b.n_alts, P->solver);
+    const int nc = std::min(most, std::max(1, int(std::ceil(most * share))));
     const size_t need = shape_smem(P->cfg.threads, P->solver, b.n_alts, nc);
     if (nc * b.n_alts > P->cfg.threads || need > ctx->max_smem)
       return set_err(ctx, GITM_ERR_ARG, "nAlts %d does not fit a CTA of %d threads", b.n_alts,
@@ -559,8 +579,9 @@ static int plan_common(GitmVertPlan* P, const double* const* alt, const double* 
                            cudaMemcpyHostToDevice));
   CUDA_TRY(ctx, cudaMalloc(&P->d_status, std::max<int64_t>(P->n_cols_total, 1) * sizeof(uint32_t)));
   CUDA_TRY(ctx, cudaMemset(P->d_status, 0, std::max<int64_t>(P->n_cols_total, 1) * sizeof(uint32_t)));
-  // default launch shape: 256 threads (no register spills), as many columns as fit
-  P->cfg.threads = 256;
+  // default launch shape: the tile kernel where it is built (Rusanov on GITM
+  // arrays), else 256 threads (no register spills), as many columns as fit
+  P->cfg.threads = (P->io == 0 && P->solver == GITM_SOLVER_RUSANOV) ? TILE_THREADS : 256;
   P->cfg.cols_per_cta = 0;
   P->cfg.steps_per_launch = 1;
   P->cfg.ctas_per_sm = 0;
@@ -572,7 +593,6 @@ static void plan_free(GitmVertPlan* P) {
   cudaFree(P->d_adj_tiles);
   cudaFree(P->d_save_tiles);
   cudaFree(P->d_adj_scratch);
-  cudaFree(P->d_save_scratch);
   cudaFree(P->d_bars);
   cudaFree(P->d_scratch);
   cudaFree(P->d_members);
@@ -882,7 +902,7 @@ constexpr int kAdjThreads = ADJ_THREADS;
 static int adjoint_prepare(GitmVertPlan* P) {
   GitmVertCtx* ctx = P->ctx;
   if (P->adj_ready) return GITM_OK;
-  const int T = kAdjThreads, TS = SAVE_THREADS;
+  const int T = kAdjThreads;
   P->adj_tiles.clear();
   P->save_tiles.clear();
   P->adj_smem = 0;
@@ -909,13 +929,19 @@ static int adjoint_prepare(GitmVertPlan* P) {
     P->adj_nc_max = std::max(P->adj_nc_max, nc);
     P->adj_per_max = std::max(P->adj_per_max, adj_state_doubles(nA));
     cut(P->adj_tiles, m, b.n_cols, nc);
-    // the saving step kernel: columns per CTA of the forward layout
-    int ns = std::max(1, std::min(TS / nA, TS / 32));
-    while (ns > 1 && smem_bytes(nA, ns) > ctx->max_smem) --ns;
-    if (nA > TS || smem_bytes(nA, ns) > ctx->max_smem)
-      return set_err(ctx, GITM_ERR_UNSUPPORTED, "saving step: nAlts %d does not fit a CTA of %d threads", nA, TS);
-    P->save_smem = std::max(P->save_smem, smem_bytes(nA, ns));
-    cut(P->save_tiles, m, b.n_cols, ns);
+  }
+  // the saving step: the tile kernel's own tiles
+  {
+    const GitmLaunchConfig cfg{TILE_THREADS, 0, 1, 0};
+    std::vector<std::pair<int64_t, int>> full;
+    for (const GitmColumnBatch& b : P->host_members)
+      full.push_back({b.n_cols, cols_per_cta(ctx, cfg, b.n_alts, P->solver)});
+    const double share = tile_share(ctx, full);
+    for (int m = 0; m < P->n_members; ++m) {
+      const int ns = std::min(full[m].second, std::max(1, int(std::ceil(full[m].second * share))));
+      P->save_smem = std::max(P->save_smem, tile_smem_bytes(P->host_members[m].n_alts, ns));
+      cut(P->save_tiles, m, P->host_members[m].n_cols, ns);
+    }
   }
   if (P->adj_tiles.empty()) {
     P->adj_ready = true;
@@ -936,21 +962,12 @@ static int adjoint_prepare(GitmVertPlan* P) {
     return set_err(ctx, GITM_ERR_NOMEM, "adjoint: cannot allocate the stage-state scratch");
   }
   CUDA_TRY(ctx, cudaMalloc(&P->d_bars, std::max(1, P->n_members) * sizeof(GitmColumnAdjoint)));
-  // the saving step kernel: its own tiles, the forward layout
-  const void* sfn = kernel_for(0, GITM_SOLVER_RUSANOV, SAVE_THREADS, plan_nalts(P), true);
-  if (!sfn) return set_err(ctx, GITM_ERR_ARG, "the saving step kernel is not built");
-  CUDA_TRY(ctx, cudaFuncSetAttribute(sfn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(ctx->max_smem)));
-  int sper = 0;
-  CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&sper, sfn, TS, P->save_smem));
-  sper = std::max(sper, 1);
-  P->save_grid = int(std::min<size_t>(P->save_tiles.size(), size_t(sper) * ctx->num_sms));
+  if (!kernel_for(0, GITM_SOLVER_RUSANOV, TILE_THREADS, plan_nalts(P), true))
+    return set_err(ctx, GITM_ERR_ARG, "the saving step kernel is not built");
+  P->save_grid = int(std::min<size_t>(P->save_tiles.size(), size_t(ctx->num_sms)));
   CUDA_TRY(ctx, cudaMalloc(&P->d_save_tiles, P->save_tiles.size() * sizeof(Tile)));
   CUDA_TRY(ctx, cudaMemcpy(P->d_save_tiles, P->save_tiles.data(), P->save_tiles.size() * sizeof(Tile),
                            cudaMemcpyHostToDevice));
-  if (cudaMalloc(&P->d_save_scratch, size_t(P->save_grid) * NF * TS * sizeof(double)) != cudaSuccess) {
-    cudaGetLastError();
-    return set_err(ctx, GITM_ERR_NOMEM, "adjoint: cannot allocate the saving step's scratch");
-  }
   P->adj_ready = true;
   return GITM_OK;
 }
@@ -991,14 +1008,13 @@ extern "C" int gitm_vert_plan_advance_saving(GitmVertPlan* P, double dt, double*
   kp.n_steps = 1;
   kp.dt = dt;
   kp.status = P->d_status;
-  kp.scratch = P->d_save_scratch;
   kp.prm = ctx->params;
   kp.save = states;
   kp.save_ncols = P->n_cols_total;
   kp.save_per = P->adj_per_max;
   void* args[] = {&kp};
-  CUDA_TRY(ctx, cudaLaunchKernel(kernel_for(0, GITM_SOLVER_RUSANOV, SAVE_THREADS, plan_nalts(P), true), dim3(P->save_grid), dim3(SAVE_THREADS), args, P->save_smem,
-                                 static_cast<cudaStream_t>(stream)));
+  CUDA_TRY(ctx, cudaLaunchKernel(kernel_for(0, GITM_SOLVER_RUSANOV, TILE_THREADS, plan_nalts(P), true), dim3(P->save_grid),
+                                 dim3(TILE_THREADS), args, P->save_smem, static_cast<cudaStream_t>(stream)));
   return GITM_OK;
 }
 

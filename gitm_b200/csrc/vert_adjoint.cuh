@@ -58,9 +58,8 @@ __host__ __device__ inline AdjLayout make_adj_layout(int nAlts) {
 
 constexpr int ADJ_NSTATE = 6;    // gathered state, X0, X1, X2, X3, X4
 // threads per CTA of the adjoint kernel (2 columns of 50 cells per CTA; 64
-// threads with one column measured 3 % slower) and of the saving step kernel
+// threads with one column measured 3 % slower)
 constexpr int ADJ_THREADS = 128;
-constexpr int SAVE_THREADS = 128;
 // The stage adjoint's shares that cross a warp boundary inside a column: per
 // boundary (lane 31 of warp b | lane 0 of warp b+1) and swept field, the
 // value and slope shares to the right cell and to the left cell.

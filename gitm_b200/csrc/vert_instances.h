@@ -1,7 +1,7 @@
 // vert_instances.h -- the step-kernel instantiations the library is built with.
 //
-// X(id, IO, NT, MINB, ACC_GLOBAL, SOLVER, SAVE, NA, OG): vert_step_kernel<IO,
-// NT, MINB, ACC_GLOBAL, SOLVER, SAVE, NA, OG> (vert_kernel.cuh).  Each entry is compiled
+// X(id, IO, NT, MINB, ACC_GLOBAL, SOLVER, NA, OG): vert_step_kernel<IO, NT,
+// MINB, ACC_GLOBAL, SOLVER, NA, OG> (vert_kernel.cuh).  Each entry is compiled
 // in a translation unit of its own (vert_instance.cu, built once per entry
 // with -DGV_ID=id -DGV_IO=... by gitm_b200/build.py, which reads this list):
 // instantiated side by side in one unit, the compiler kept arrays of the
@@ -18,44 +18,45 @@
 // (the AUSM solver's 384-thread shape).
 //
 // GV_TILE_INSTANCES lists the 512-thread shape of the Rusanov solver on GITM
-// arrays, a kernel of its own (vert_tile.cuh): T(id, SAVE, NA).
+// arrays, a kernel of its own (vert_tile.cuh): T(id, SAVE, NA).  SAVE: the
+// step that keeps its stage states for the adjoint.
 #pragma once
 
 #include "vert_common.cuh"
 
 #define GV_STEP_INSTANCES(X)                                  \
-  X(rus0_t128, 0, 128, 3, true, 0, false, 0, false)           \
-  X(rus0_t160, 0, 160, 2, true, 0, false, 0, false)           \
-  X(rus0_t192, 0, 192, 2, true, 0, false, 0, false)           \
-  X(rus0_t256, 0, 256, 1, false, 0, false, 0, false)          \
-  X(rus0_t320, 0, 320, 1, false, 0, false, 0, false)          \
-  X(rus0_t384, 0, 384, 1, false, 0, false, 0, false)          \
-  X(rus1_t128, 1, 128, 3, true, 0, false, 0, false)           \
-  X(rus1_t160, 1, 160, 2, true, 0, false, 0, false)           \
-  X(rus1_t192, 1, 192, 2, true, 0, false, 0, false)           \
-  X(rus1_t256, 1, 256, 1, false, 0, false, 0, false)          \
-  X(rus1_t320, 1, 320, 1, false, 0, false, 0, false)          \
-  X(rus1_t384, 1, 384, 1, false, 0, false, 0, false)          \
-  X(ausm0_t128, 0, 128, 2, true, 1, false, 0, false)          \
-  X(ausm0_t256, 0, 256, 1, false, 1, false, 0, false)         \
-  X(ausm1_t128, 1, 128, 2, true, 1, false, 0, false)          \
-  X(ausm1_t256, 1, 256, 1, false, 1, false, 0, false)         \
-  X(rus0_t128_save, 0, 128, 3, true, 0, true, 0, false)       \
-  X(rus0_t128_n50, 0, 128, 3, true, 0, false, 50, false)      \
-  X(rus0_t192_n50, 0, 192, 2, true, 0, false, 50, false)      \
-  X(rus0_t256_n50, 0, 256, 1, false, 0, false, 50, false)     \
-  X(rus0_t384_n50, 0, 384, 1, false, 0, false, 50, false)     \
-  X(ausm0_t128_n50, 0, 128, 2, true, 1, false, 50, false)     \
-  X(ausm0_t256_n50, 0, 256, 1, false, 1, false, 50, false)    \
-  X(rus0_t128_save_n50, 0, 128, 3, true, 0, true, 50, false)  \
-  X(ausm0_t384_og_n50, 0, 384, 1, true, 1, false, 50, true)
+  X(rus0_t128, 0, 128, 3, true, 0, 0, false)                  \
+  X(rus0_t160, 0, 160, 2, true, 0, 0, false)                  \
+  X(rus0_t192, 0, 192, 2, true, 0, 0, false)                  \
+  X(rus0_t256, 0, 256, 1, false, 0, 0, false)                 \
+  X(rus0_t320, 0, 320, 1, false, 0, 0, false)                 \
+  X(rus0_t384, 0, 384, 1, false, 0, 0, false)                 \
+  X(rus1_t128, 1, 128, 3, true, 0, 0, false)                  \
+  X(rus1_t160, 1, 160, 2, true, 0, 0, false)                  \
+  X(rus1_t192, 1, 192, 2, true, 0, 0, false)                  \
+  X(rus1_t256, 1, 256, 1, false, 0, 0, false)                 \
+  X(rus1_t320, 1, 320, 1, false, 0, 0, false)                 \
+  X(rus1_t384, 1, 384, 1, false, 0, 0, false)                 \
+  X(ausm0_t128, 0, 128, 2, true, 1, 0, false)                 \
+  X(ausm0_t256, 0, 256, 1, false, 1, 0, false)                \
+  X(ausm1_t128, 1, 128, 2, true, 1, 0, false)                 \
+  X(ausm1_t256, 1, 256, 1, false, 1, 0, false)                \
+  X(rus0_t128_n50, 0, 128, 3, true, 0, 50, false)             \
+  X(rus0_t192_n50, 0, 192, 2, true, 0, 50, false)             \
+  X(rus0_t256_n50, 0, 256, 1, false, 0, 50, false)            \
+  X(rus0_t384_n50, 0, 384, 1, false, 0, 50, false)            \
+  X(ausm0_t128_n50, 0, 128, 2, true, 1, 50, false)            \
+  X(ausm0_t256_n50, 0, 256, 1, false, 1, 50, false)           \
+  X(ausm0_t384_og_n50, 0, 384, 1, true, 1, 50, true)
 
 #define GV_TILE_INSTANCES(T)     \
   T(tile, false, 0)              \
-  T(tile_n50, false, 50)
+  T(tile_n50, false, 50)         \
+  T(tile_save, true, 0)          \
+  T(tile_save_n50, true, 50)
 
 namespace gv {
-#define GV_DECLARE_INSTANCE(id, IO, NT, MINB, ACC, SOLVER, SAVE, NA, OG) \
+#define GV_DECLARE_INSTANCE(id, IO, NT, MINB, ACC, SOLVER, NA, OG) \
   const void* step_kernel_##id();                                \
   cudaError_t step_consts_##id(const Consts& k);
 GV_STEP_INSTANCES(GV_DECLARE_INSTANCE)

@@ -762,7 +762,7 @@ struct KParams {
                       // (ACC_GLOBAL), then with OG the Orig of the tile's columns
   int64_t scratch_per_cta;  // doubles of one CTA's slot (OG kernels)
   GitmVertParams prm;
-  // SAVE kernels (one step per launch): the gathered state and the
+  // the saving tile kernel (one step per launch): the gathered state and the
   // post-boundary stage states X0..X4 of every column, state s of global
   // column c at save[(s * save_ncols + c) * save_per], for the adjoint
   double* save;
@@ -781,7 +781,7 @@ struct KParams {
 // OG (with ACC_GLOBAL): Orig lives in the CTA's slot of global scratch after
 // the accumulators (coalesced, L2-resident, read-only within a step), so a
 // column needs 8 KB less shared memory and more columns share an SM.
-template <int IO, int NT, int MINB, bool ACC_GLOBAL, int SOLVER, bool SAVE = false, int NA = 0, bool OG = false>
+template <int IO, int NT, int MINB, bool ACC_GLOBAL, int SOLVER, int NA = 0, bool OG = false>
 __global__ void __launch_bounds__(NT, MINB) vert_step_kernel(const KParams kp) {
   static_assert(!OG || ACC_GLOBAL, "Orig in global scratch goes with the accumulators there");
   extern __shared__ double sm[];
@@ -826,19 +826,6 @@ __global__ void __launch_bounds__(NT, MINB) vert_step_kernel(const KParams kp) {
     };
     auto gidx = [&](int f, int g, int cl) -> int64_t {
       return (int64_t(f) * G + g) * ncols + tile.c0 + cl;
-    };
-    // SAVE: copies the current stage buffer (state and passive cells) of
-    // every column of the tile to saved state s
-    auto save_state = [&](int s) {
-      if constexpr (SAVE) {
-        const int per = NF * G + NPAS * NPC;
-        const int xo = cur ? L.X1 : L.X0;
-        for (int cl = 0; cl < nc; ++cl) {
-          const double* src = sm + size_t(L.stride) * cl + xo;
-          double* dst = kp.save + (int64_t(s) * kp.save_ncols + M.col_offset + tile.c0 + cl) * kp.save_per;
-          for (int r = tid; r < per; r += NT) dst[r] = src[r];
-        }
-      }
     };
     // set_vertical_bcs for every column of the tile: the lower and upper
     // halves of a column go to different warps when there are enough
@@ -997,10 +984,6 @@ __global__ void __launch_bounds__(NT, MINB) vert_step_kernel(const KParams kp) {
       }
     }
     __syncthreads();  // @phase 0
-    if constexpr (SAVE) {
-      save_state(0);
-      __syncthreads();  // the boundary pass rewrites what was just saved
-    }
 
     // per-item constants for the step
     double eddy = 0.0, ivup = 0.0;
@@ -1020,7 +1003,6 @@ __global__ void __launch_bounds__(NT, MINB) vert_step_kernel(const KParams kp) {
       // ---------------------------------------------------- first BC pass
       boundaries();
       __syncthreads();  // @phase 1
-      save_state(1);
       // Orig = state (vertical_solver_rusanov.f90:95-100); read first in
       // phase B, after the barrier that ends phase A
       {
@@ -1147,7 +1129,6 @@ __global__ void __launch_bounds__(NT, MINB) vert_step_kernel(const KParams kp) {
         // set_vertical_bcs on the updated state (:166,236,306,368)
         boundaries();
         __syncthreads();  // @phase 1
-        save_state(2 + k);
       }
 
       // ---------------------------------------------------- store / reload

@@ -549,7 +549,7 @@ __device__ __forceinline__ double tile_heated(const GitmColumnBatch& b, double t
 }
 
 // ------------------------------------------------------------ the kernel
-// kp.scratch is not used.  SAVE as in vert_step_kernel.
+// kp.scratch is not used.  SAVE: see KParams::save.
 template <int NA, bool SAVE>
 __global__ void __launch_bounds__(TILE_THREADS, 1) vert_tile_kernel(const KParams kp) {
   extern __shared__ double sm[];
