@@ -136,6 +136,7 @@ static void fill_consts(Consts& k) {
   for (int s = 0; s < NS; ++s) {
     k.mass[s] = mass[s];
     k.log_mass[s] = std::log(mass[s]);
+    k.inv_mass[s] = 1.0 / mass[s];
     k.log_kb = std::log(KB);
     k.k_over_m[s] = KB / mass[s];
     k.inv_vib2[s] = 1.0 / (vib[s] - 2);

@@ -61,6 +61,7 @@ enum AusmGridCoef : int {
 struct Consts {
   double mass[NS];
   double log_mass[NS];
+  double inv_mass[NS];
   double k_over_m[NS];
   double inv_vib2[NS];           // 1 / (Vibration - 2)
   double kc[NS][NS];             // 1e-2 k / (Mass_i Diff0_ij): friction coefficient

@@ -490,21 +490,72 @@ static __device__ __noinline__ bool friction_singular(double dt, const double* n
 }
 
 // calc_neutral_friction (calc_neutral_friction.f90:47-106) for one cell:
-// solves (I + dt C) v = w in place.  C_ij = 1e-2 k / (M_i D0_ij) n_j
-// T^(1 - DiffExp_ij) (the NDensity factors of the reference cancel).  Row i
-// times the species' mass density M_i n_i makes the matrix symmetric: the
-// pair coefficient 1e-2 k / D0 T^(1 - DiffExp) takes six values, one per
-// distinct exponent, and W_ij = dt (pair coefficient) n_i n_j.  With
-// S = diag(M_i n_i + sum_j W_ij) - W (diagonally dominant, so no pivoting)
-// the LDL^T elimination holds 21 values instead of 36 and takes 65
-// multiply-adds instead of 85; off the diagonal it only adds positive terms
-// (with the direct increments of rusanov_cell: the 1 degree globe's 16 steps
-// 59.3 -> 56.3 ms, error against 64-bit arithmetic 1.3e-12 -> 5e-13; the AUSM
-// solver at 2.5 degrees, 4 steps, 11.45 -> 10.60 ms).
-// mn[s] = M_s n_s.  A non-finite density or temperature takes the reference's
-// row test, which sets GITM_ST_LU_SINGULAR in *st (when st is given); the
-// solve goes on, its results non-finite.  WARP: whole warps call it, and no
-// branch splits them (the caller's next instruction needs the warp converged).
+// (I + dt C) v = w with C_ij = 1e-2 k / (M_i D0_ij) n_j T^(1 - DiffExp_ij)
+// (the NDensity factors of the reference cancel).  Row i times the species'
+// mass density M_i n_i makes the matrix symmetric: the pair coefficient
+// 1e-2 k / D0 T^(1 - DiffExp) takes six values, one per distinct exponent,
+// and W_ij = dt (pair coefficient) n_i n_j.  S = diag(M_i n_i + sum_j W_ij) -
+// W is diagonally dominant, so the LDL^T elimination needs no pivoting; it
+// holds 21 values instead of 36 and takes 65 multiply-adds instead of 85, and
+// off the diagonal it only adds positive terms (with the direct increments of
+// rusanov_cell: the 1 degree globe's 16 steps 59.3 -> 56.3 ms, error against
+// 64-bit arithmetic 1.3e-12 -> 5e-13; the AUSM solver at 2.5 degrees, 4
+// steps, 11.45 -> 10.60 ms).  factor: pe[e] = dt (pair coefficient), mn[s] =
+// M_s n_s; solve: b = M n w in, v out.
+struct FrictionLdl {
+  double d[NS];      // reciprocal pivots
+  double w[NS][NS];  // below the diagonal
+  __device__ __forceinline__ void factor(const double (&ns)[NS], const double (&mn)[NS], const double (&pe)[NS]) {
+#pragma unroll
+    for (int r = 0; r < NS; ++r) d[r] = mn[r];
+#pragma unroll
+    for (int r = 1; r < NS; ++r)
+#pragma unroll
+      for (int q = 0; q < r; ++q) {
+        w[r][q] = (ns[r] * ns[q]) * pe[exp_index(r, q)];
+        d[r] += w[r][q];
+        d[q] += w[r][q];
+      }
+  }
+  // the elimination, on one right-hand side as well
+  __device__ __forceinline__ void eliminate(double (&b)[NS]) {
+#pragma unroll
+    for (int p = 0; p < NS; ++p) {
+      d[p] = rcp_nr(d[p]);
+#pragma unroll
+      for (int r = p + 1; r < NS; ++r) {
+        const double l = w[r][p] * d[p];
+#pragma unroll
+        for (int q = p + 1; q < r; ++q) w[r][q] = fma(l, w[q][p], w[r][q]);
+        d[r] = fma(-l, w[r][p], d[r]);
+        b[r] = fma(l, b[p], b[r]);
+      }
+    }
+  }
+  __device__ __forceinline__ void forward(double (&b)[NS]) const {
+#pragma unroll
+    for (int p = 0; p < NS; ++p) {
+      const double t = b[p] * d[p];
+#pragma unroll
+      for (int r = p + 1; r < NS; ++r) b[r] = fma(w[r][p], t, b[r]);
+    }
+  }
+  __device__ __forceinline__ void back(double (&b)[NS]) const {
+#pragma unroll
+    for (int r = NS - 1; r >= 0; --r) {
+      double sum = b[r];
+#pragma unroll
+      for (int q = r + 1; q < NS; ++q) sum = fma(w[q][r], b[q], sum);
+      b[r] = sum * d[r];
+    }
+  }
+};
+
+// The friction solve in place of wv.  A non-finite density or temperature
+// takes the reference's row test, which sets GITM_ST_LU_SINGULAR in *st (when
+// st is given); the solve goes on, its results non-finite.  WARP: whole warps
+// call it, and no branch splits them (the caller's next instruction needs the
+// warp converged).
 template <bool WARP = false>
 __device__ __forceinline__ void friction_solve(double dt, const double (&ns)[NS], const double (&mn)[NS], double T,
                                                double (&wv)[NS], uint32_t* st = nullptr) {
@@ -531,38 +582,12 @@ __device__ __forceinline__ void friction_solve(double dt, const double (&ns)[NS]
   }
 #pragma unroll
   for (int e = 0; e < NS; ++e) pw[e] = (dt * c_k.kpair[e]) * pw[e];
-  double d[NS], w[NS][NS];  // the diagonal; W below it
-#pragma unroll
-  for (int r = 0; r < NS; ++r) d[r] = mn[r];
-#pragma unroll
-  for (int r = 1; r < NS; ++r)
-#pragma unroll
-    for (int q = 0; q < r; ++q) {
-      w[r][q] = (ns[r] * ns[q]) * pw[exp_index(r, q)];
-      d[r] += w[r][q];
-      d[q] += w[r][q];
-    }
 #pragma unroll
   for (int r = 0; r < NS; ++r) wv[r] *= mn[r];
-#pragma unroll
-  for (int p = 0; p < NS; ++p) {
-    d[p] = rcp_nr(d[p]);
-#pragma unroll
-    for (int r = p + 1; r < NS; ++r) {
-      const double l = w[r][p] * d[p];
-#pragma unroll
-      for (int q = p + 1; q < r; ++q) w[r][q] = fma(l, w[q][p], w[r][q]);
-      d[r] = fma(-l, w[r][p], d[r]);
-      wv[r] = fma(l, wv[p], wv[r]);
-    }
-  }
-#pragma unroll
-  for (int r = NS - 1; r >= 0; --r) {
-    double sum = wv[r];
-#pragma unroll
-    for (int q = r + 1; q < NS; ++q) sum = fma(w[q][r], wv[q], sum);
-    wv[r] = sum * d[r];
-  }
+  FrictionLdl m;
+  m.factor(ns, mn, pw);
+  m.eliminate(wv);
+  m.back(wv);
 }
 
 // GradLogConS at cell i (vertical_solver_rusanov.f90:506-543,
@@ -668,7 +693,6 @@ __device__ __forceinline__ void rusanov_cell(ColCtx c, int i, const GitmVertPara
     const double pg = fma(T, gL, gT * (1.0 + prm.thermal_diff_coef[s]));
     wv[s] = fma(-dt, fma(c_k.k_over_m[s], pg, Ws * gW), fma(Ws, keep, common) + dW);
   }
-  const double LR = c.x(F_LRHO, i);
   double ns[NS], mn[NS];
   exp_n<NS, WARP>(nl, ns);
   {
@@ -676,7 +700,7 @@ __device__ __forceinline__ void rusanov_cell(ColCtx c, int i, const GitmVertPara
 #pragma unroll
     for (int s = 0; s < NS; ++s) rho[0] = fma(c_k.mass[s], ns[s], rho[0]);
     log_n<1, WARP>(rho, lr);
-    emit(F_LRHO, lr[0] - LR);
+    emit(F_LRHO, lr[0] - c.x(F_LRHO, i));
   }
   // NS = exp(LogNS), 1 / Rho (:466-467)
   double ir;
@@ -684,7 +708,7 @@ __device__ __forceinline__ void rusanov_cell(ColCtx c, int i, const GitmVertPara
     double l7[NS + 1], e7[NS + 1];
 #pragma unroll
     for (int s = 0; s < NS; ++s) l7[s] = c.x(F_LNS + s, i);
-    l7[NS] = -LR;
+    l7[NS] = -c.x(F_LRHO, i);
     exp_n<NS + 1, WARP>(l7, e7);
 #pragma unroll
     for (int s = 0; s < NS; ++s) {
@@ -764,10 +788,12 @@ struct KParams {
   GitmVertParams prm;
   // the saving tile kernel (one step per launch): the gathered state and the
   // post-boundary stage states X0..X4 of every column, state s of global
-  // column c at save[(s * save_ncols + c) * save_per], for the adjoint
+  // column c at save[(s * save_ncols + c - save_c0) * save_per], for the adjoint
   double* save;
   int64_t save_ncols;
+  int64_t save_c0;  // the plan's column the buffer starts with
   int save_per;
+  int no_store;     // the stage states alone: the members' arrays stay as they are
 };
 
 // IO = 0: GITM arrays (advance_vertical gather/scatter);
@@ -831,11 +857,9 @@ __global__ void __launch_bounds__(NT, MINB) vert_step_kernel(const KParams kp) {
     // halves of a column go to different warps when there are enough
     auto boundaries = [&]() {
       constexpr int nw = NT / 32;
-      if (2 * nc <= nw) {
-        if (wid < 2 * nc) bc_column(ctx(wid >> 1), prm, lane, &sst[wid >> 1], 1 + (wid & 1));
-      } else {
-        for (int cl = wid; cl < nc; cl += nw) bc_column(ctx(cl), prm, lane, &sst[cl], 3);
-      }
+      const int halves = (2 * nc <= nw) ? 1 : 0;
+      for (int t = wid; t < (nc << halves); t += nw)
+        bc_column(ctx(t >> halves), prm, lane, &sst[t >> halves], halves ? 1 + (t & 1) : 3);
     };
 
     if (tid < nc) {
@@ -1000,34 +1024,36 @@ __global__ void __launch_bounds__(NT, MINB) vert_step_kernel(const KParams kp) {
           ivup = M.mv.ivel[gidx(2, my_i + 1, my_cl)];
         }
       }
-      // ---------------------------------------------------- first BC pass
-      boundaries();
-      __syncthreads();  // @phase 1
-      // Orig = state (vertical_solver_rusanov.f90:95-100); read first in
-      // phase B, after the barrier that ends phase A
-      {
-        const int xo = cur ? L.X1 : L.X0;  // X and its passive cells are contiguous
-        const int per = NF * G + NPAS * NPC;
-        for (int w = tid; w < nc * per; w += NT) {
-          const int cl = w / per, r = w - cl * per;
-          double* col = sm + size_t(L.stride) * cl;
-          if constexpr (OG) {
-            const double v = col[xo + r];
-            ogb[size_t(cl) * operc + r] = v;
-            if (r >= NF * G) {
-              col[L.OGH + NF * 4 + (r - NF * G)] = v;
+      // one copy of each phase: the boundary pass of every stage state (the
+      // first one, then after each stage) stands at the head of the loop
+#pragma unroll 1
+      for (int k = 0;; ++k) {
+        // set_vertical_bcs (:95,166,236,306,368)
+        boundaries();
+        __syncthreads();  // @phase 1
+        if (k == 4) break;
+        // Orig = state (vertical_solver_rusanov.f90:95-100); read first in
+        // phase B, after the barrier that ends phase A
+        if (k == 0) {
+          const int xo = cur ? L.X1 : L.X0;  // X and its passive cells are contiguous
+          const int per = NF * G + NPAS * NPC;
+          for (int w = tid; w < nc * per; w += NT) {
+            const int cl = w / per, r = w - cl * per;
+            double* col = sm + size_t(L.stride) * cl;
+            if constexpr (OG) {
+              const double v = col[xo + r];
+              ogb[size_t(cl) * operc + r] = v;
+              if (r >= NF * G) {
+                col[L.OGH + NF * 4 + (r - NF * G)] = v;
+              } else {
+                const int f = r / G, g = r - f * G;
+                if (g < 2 || g >= nA + 2) col[L.OGH + f * 4 + (g < 2 ? g : g - nA)] = v;
+              }
             } else {
-              const int f = r / G, g = r - f * G;
-              if (g < 2 || g >= nA + 2) col[L.OGH + f * 4 + (g < 2 ? g : g - nA)] = v;
+              col[L.O + r] = col[xo + r];
             }
-          } else {
-            col[L.O + r] = col[xo + r];
           }
         }
-      }
-
-#pragma unroll 1
-      for (int k = 0; k < 4; ++k) {
         // -------------------------------------------------- phase A
         if constexpr (SOLVER == GITM_SOLVER_AUSM) {
           // log T and the hydrostatic prefix sum of each column, then the 32
@@ -1126,9 +1152,6 @@ __global__ void __launch_bounds__(NT, MINB) vert_step_kernel(const KParams kp) {
         }
         cur ^= 1;
         __syncthreads();  // @phase 3
-        // set_vertical_bcs on the updated state (:166,236,306,368)
-        boundaries();
-        __syncthreads();  // @phase 1
       }
 
       // ---------------------------------------------------- store / reload

@@ -617,7 +617,7 @@ __global__ void __launch_bounds__(TILE_THREADS, 1) vert_tile_kernel(const KParam
           const int f = r / G;
           const double* col = cols + size_t(L.stride) * cl;
           const double v = (f < NF) ? col[L.X0 + f * L.P + (r - f * G)] : col[L.XP0 + r - NF * G];
-          kp.save[(int64_t(s) * kp.save_ncols + M.col_offset + tile.c0 + cl) * kp.save_per + r] = v;
+          kp.save[(int64_t(s) * kp.save_ncols + M.col_offset + tile.c0 + cl - kp.save_c0) * kp.save_per + r] = v;
         }
       }
     };
@@ -911,7 +911,8 @@ __global__ void __launch_bounds__(TILE_THREADS, 1) vert_tile_kernel(const KParam
 
     // ---------------------------------------------------------- store
     // scatter, advance_vertical.f90:163-217
-    for (int w = tid; w < nc * G; w += TILE_THREADS) {
+    const bool dry = SAVE && kp.no_store != 0;
+    for (int w = tid; w < nc * G && !dry; w += TILE_THREADS) {
       const int g = w / nc, cl = w - g * nc, i = g - 1;
       ColCtx c = ctx(cl);
       if (prm.compute_coefficients) {
@@ -972,6 +973,7 @@ __global__ void __launch_bounds__(TILE_THREADS, 1) vert_tile_kernel(const KParam
       const int64_t gcol = M.col_offset + tile.c0 + tid;
       uint32_t w = sst[tid];
       if (sfrozen[tid]) w |= GITM_ST_NEG_DENSITY;
+      if (dry) w &= GITM_ST_NEG_DENSITY | GITM_ST_NEG_ION_TOP;  // what stops a gather or a boundary pass
       if (w) kp.status[gcol] |= w;
     }
     __syncthreads();
