@@ -85,11 +85,15 @@ struct GitmVertPlan {
   std::vector<Tile> adj_tiles;
   Tile* d_adj_tiles = nullptr;
   size_t adj_smem = 0;
-  int adj_grid = 0, adj_nc_max = 0, adj_per_max = 0;
-  size_t adj_scratch_per_cta = 0;
+  int adj_grid = 0, adj_per_max = 0;
   double* d_adj_scratch = nullptr;
   GitmColumnAdjoint* d_bars = nullptr;
   // the saving step kernel (its own tiles and persistent grid)
+  // tile ranges whose stage states a call without saved ones forms and
+  // reverses together, and their buffer
+  struct AdjChunk { int save0, save1, adj0, adj1; int64_t c0, n; };
+  std::vector<AdjChunk> adj_chunks;
+  double* d_adj_states = nullptr;
   std::vector<Tile> save_tiles;
   Tile* d_save_tiles = nullptr;
   int save_grid = 0;
@@ -594,6 +598,7 @@ static void plan_free(GitmVertPlan* P) {
   cudaFree(P->d_adj_tiles);
   cudaFree(P->d_save_tiles);
   cudaFree(P->d_adj_scratch);
+  cudaFree(P->d_adj_states);
   cudaFree(P->d_bars);
   cudaFree(P->d_scratch);
   cudaFree(P->d_members);
@@ -899,6 +904,40 @@ extern "C" int gitm_vert_advance_native(GitmVertCtx* ctx, const GitmColumnBatch*
 // ------------------------------------------------------------------ adjoint
 constexpr int kAdjThreads = ADJ_THREADS;
 
+// The tile ranges and the buffer of a call without saved states: about five
+// rounds of the adjoint kernel's grid at a time (2,960 columns of 50
+// altitudes, 157 MB), whole tiles of both kernels.
+static int adjoint_chunks(GitmVertPlan* P, int64_t columns) {
+  GitmVertCtx* ctx = P->ctx;
+  if (!P->adj_chunks.empty()) return GITM_OK;
+  std::vector<GitmVertPlan::AdjChunk> out;
+  size_t s = 0, a = 0;
+  int64_t off = 0, most = 0;
+  for (int m = 0; m < P->n_members; ++m) {
+    const int64_t n_cols = P->host_members[m].n_cols;
+    if (n_cols == 0) continue;
+    const int64_t both = int64_t(P->save_tiles[s].nc) * P->adj_tiles[a].nc;  // a boundary of both tilings
+    const int64_t step = std::max<int64_t>(1, columns / both) * both;
+    for (int64_t c0 = 0; c0 < n_cols; c0 += step) {
+      const int64_t c1 = std::min(n_cols, c0 + step);
+      GitmVertPlan::AdjChunk ch{int(s), 0, int(a), 0, off + c0, c1 - c0};
+      while (s < P->save_tiles.size() && P->save_tiles[s].member == m && P->save_tiles[s].c0 < c1) ++s;
+      while (a < P->adj_tiles.size() && P->adj_tiles[a].member == m && P->adj_tiles[a].c0 < c1) ++a;
+      ch.save1 = int(s);
+      ch.adj1 = int(a);
+      most = std::max(most, ch.n);
+      out.push_back(ch);
+    }
+    off += n_cols;
+  }
+  if (cudaMalloc(&P->d_adj_states, size_t(ADJ_NSTATE) * most * P->adj_per_max * sizeof(double)) != cudaSuccess) {
+    cudaGetLastError();
+    return set_err(ctx, GITM_ERR_NOMEM, "adjoint: cannot allocate the stage states of %lld columns", (long long)most);
+  }
+  P->adj_chunks = std::move(out);
+  return GITM_OK;
+}
+
 // Tiles, persistent grid and scratch of the adjoint kernel for the plan.
 static int adjoint_prepare(GitmVertPlan* P) {
   GitmVertCtx* ctx = P->ctx;
@@ -907,7 +946,6 @@ static int adjoint_prepare(GitmVertPlan* P) {
   P->adj_tiles.clear();
   P->save_tiles.clear();
   P->adj_smem = 0;
-  P->adj_nc_max = 1;
   P->adj_per_max = 0;
   P->save_smem = 0;
   auto cut = [](std::vector<Tile>& out, int m, int64_t n_cols, int nc) {
@@ -927,7 +965,6 @@ static int adjoint_prepare(GitmVertPlan* P) {
     if (nA > T || adj_smem_bytes(nA, nc) > ctx->max_smem)
       return set_err(ctx, GITM_ERR_UNSUPPORTED, "adjoint: nAlts %d does not fit a CTA of %d threads", nA, T);
     P->adj_smem = std::max(P->adj_smem, adj_smem_bytes(nA, nc));
-    P->adj_nc_max = std::max(P->adj_nc_max, nc);
     P->adj_per_max = std::max(P->adj_per_max, adj_state_doubles(nA));
     cut(P->adj_tiles, m, b.n_cols, nc);
   }
@@ -954,13 +991,12 @@ static int adjoint_prepare(GitmVertPlan* P) {
   CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, T, P->adj_smem));
   per_sm = std::max(per_sm, 1);
   P->adj_grid = int(std::min<size_t>(P->adj_tiles.size(), size_t(per_sm) * ctx->num_sms));
-  P->adj_scratch_per_cta = size_t(ADJ_NSTATE) * P->adj_nc_max * P->adj_per_max + size_t(2) * NF * T;
   CUDA_TRY(ctx, cudaMalloc(&P->d_adj_tiles, P->adj_tiles.size() * sizeof(Tile)));
   CUDA_TRY(ctx, cudaMemcpy(P->d_adj_tiles, P->adj_tiles.data(), P->adj_tiles.size() * sizeof(Tile),
                            cudaMemcpyHostToDevice));
-  if (cudaMalloc(&P->d_adj_scratch, size_t(P->adj_grid) * P->adj_scratch_per_cta * sizeof(double)) != cudaSuccess) {
+  if (cudaMalloc(&P->d_adj_scratch, size_t(P->adj_grid) * 2 * NF * T * sizeof(double)) != cudaSuccess) {
     cudaGetLastError();
-    return set_err(ctx, GITM_ERR_NOMEM, "adjoint: cannot allocate the stage-state scratch");
+    return set_err(ctx, GITM_ERR_NOMEM, "adjoint: cannot allocate the stage-adjoint scratch");
   }
   CUDA_TRY(ctx, cudaMalloc(&P->d_bars, std::max(1, P->n_members) * sizeof(GitmColumnAdjoint)));
   if (!kernel_for(0, GITM_SOLVER_RUSANOV, TILE_THREADS, plan_nalts(P), true))
@@ -969,6 +1005,8 @@ static int adjoint_prepare(GitmVertPlan* P) {
   CUDA_TRY(ctx, cudaMalloc(&P->d_save_tiles, P->save_tiles.size() * sizeof(Tile)));
   CUDA_TRY(ctx, cudaMemcpy(P->d_save_tiles, P->save_tiles.data(), P->save_tiles.size() * sizeof(Tile),
                            cudaMemcpyHostToDevice));
+  const int rc = adjoint_chunks(P, 5 * int64_t(P->adj_grid) * P->adj_tiles[0].nc);
+  if (rc) return rc;
   P->adj_ready = true;
   return GITM_OK;
 }
@@ -990,6 +1028,30 @@ static int adjoint_checks(GitmVertPlan* P) {
   return GITM_OK;
 }
 
+// The saving step over tiles t0 .. t1 of the plan's saving tiles; the buffer
+// starts with column c0 and holds n columns per state.
+static int launch_saving(GitmVertPlan* P, double dt, int t0, int t1, double* states, int64_t c0, int64_t n, bool store,
+                         cudaStream_t st) {
+  GitmVertCtx* ctx = P->ctx;
+  KParams kp{};
+  kp.members = P->d_members;
+  kp.tiles = P->d_save_tiles + t0;
+  kp.n_tiles = t1 - t0;
+  kp.n_steps = 1;
+  kp.dt = dt;
+  kp.status = P->d_status;
+  kp.prm = ctx->params;
+  kp.save = states;
+  kp.save_ncols = n;
+  kp.save_c0 = c0;
+  kp.save_per = P->adj_per_max;
+  kp.no_store = store ? 0 : 1;
+  void* args[] = {&kp};
+  CUDA_TRY(ctx, cudaLaunchKernel(kernel_for(0, GITM_SOLVER_RUSANOV, TILE_THREADS, plan_nalts(P), true),
+                                 dim3(std::min(kp.n_tiles, P->save_grid)), dim3(TILE_THREADS), args, P->save_smem, st));
+  return GITM_OK;
+}
+
 extern "C" int gitm_vert_plan_advance_saving(GitmVertPlan* P, double dt, double* states, void* stream) {
   if (!P) return GITM_ERR_ARG;
   GitmVertCtx* ctx = P->ctx;
@@ -1001,22 +1063,8 @@ extern "C" int gitm_vert_plan_advance_saving(GitmVertPlan* P, double dt, double*
   rc = adjoint_prepare(P);
   if (rc) return rc;
   if (P->adj_tiles.empty()) return GITM_OK;
-  KParams kp{};
-  std::memset(&kp, 0, sizeof kp);
-  kp.members = P->d_members;
-  kp.tiles = P->d_save_tiles;
-  kp.n_tiles = int(P->save_tiles.size());
-  kp.n_steps = 1;
-  kp.dt = dt;
-  kp.status = P->d_status;
-  kp.prm = ctx->params;
-  kp.save = states;
-  kp.save_ncols = P->n_cols_total;
-  kp.save_per = P->adj_per_max;
-  void* args[] = {&kp};
-  CUDA_TRY(ctx, cudaLaunchKernel(kernel_for(0, GITM_SOLVER_RUSANOV, TILE_THREADS, plan_nalts(P), true), dim3(P->save_grid),
-                                 dim3(TILE_THREADS), args, P->save_smem, static_cast<cudaStream_t>(stream)));
-  return GITM_OK;
+  return launch_saving(P, dt, 0, int(P->save_tiles.size()), states, 0, P->n_cols_total, true,
+                       static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int gitm_vert_plan_adjoint(GitmVertPlan* P, const GitmColumnAdjoint* bars, double dt,
@@ -1050,20 +1098,28 @@ extern "C" int gitm_vert_plan_adjoint(GitmVertPlan* P, const GitmColumnAdjoint* 
   }
   kp.members = P->d_members;
   kp.bars = P->d_bars;
-  kp.tiles = P->d_adj_tiles;
-  kp.n_tiles = int(P->adj_tiles.size());
-  kp.nc_max = P->adj_nc_max;
   kp.per_max = P->adj_per_max;
   kp.dt = dt;
   kp.status = P->d_status;
   kp.scratch = P->d_adj_scratch;
-  kp.scratch_per_cta = P->adj_scratch_per_cta;
   kp.prm = ctx->params;
-  kp.saved = saved_states;
-  kp.saved_ncols = P->n_cols_total;
-  void* args[] = {&kp};
-  CUDA_TRY(ctx, cudaLaunchKernel((plan_nalts(P) == 50) ? adjoint_kernel_fn_n50() : adjoint_kernel_fn(), dim3(P->adj_grid),
-                                 dim3(kAdjThreads), args, P->adj_smem, st));
+  const void* fn = (plan_nalts(P) == 50) ? adjoint_kernel_fn_n50() : adjoint_kernel_fn();
+  auto launch = [&](int t0, int t1, const double* states, int64_t c0, int64_t n) -> int {
+    kp.tiles = P->d_adj_tiles + t0;
+    kp.n_tiles = t1 - t0;
+    kp.saved = states;
+    kp.saved_ncols = n;
+    kp.saved_c0 = c0;
+    void* args[] = {&kp};
+    CUDA_TRY(ctx, cudaLaunchKernel(fn, dim3(std::min(kp.n_tiles, P->adj_grid)), dim3(kAdjThreads), args, P->adj_smem, st));
+    return GITM_OK;
+  };
+  if (saved_states) return launch(0, int(P->adj_tiles.size()), saved_states, 0, P->n_cols_total);
+  for (const GitmVertPlan::AdjChunk& ch : P->adj_chunks) {
+    rc = launch_saving(P, dt, ch.save0, ch.save1, P->d_adj_states, ch.c0, ch.n, false, st);
+    if (!rc) rc = launch(ch.adj0, ch.adj1, P->d_adj_states, ch.c0, ch.n);
+    if (rc) return rc;
+  }
   return GITM_OK;
 }
 

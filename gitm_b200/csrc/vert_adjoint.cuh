@@ -6,11 +6,10 @@
 // branch (limiter case, clamp, boundary switch, max of |w|) differentiated on
 // the side the forward took.
 //
-// One CTA per tile of columns, persistent over tiles.  The CTA first re-runs
-// the step forward (gather, producers, boundaries, four stages) and saves
-// the six states it needs -- the gathered state, the post-boundary stage
-// inputs X0..X3 and the final X4 -- to a per-CTA slot of global scratch
-// (L2-resident under the persistent grid).  The reverse sweep then runs from
+// One CTA per tile of columns, persistent over tiles.  The states it needs --
+// the gathered state, the post-boundary stage inputs X0..X3 and the final X4
+// -- come from the saving step (vert_tile.cuh), run by the caller, or ahead of
+// this kernel a few thousand columns at a time.  The reverse sweep runs from
 // the scatter back to the gather:
 //   scatter^T -> bc^T(X4) -> RK combination^T -> for k = 3..0:
 //     load X_k, recompute its slopes, stage_k^T at every interior cell
@@ -87,18 +86,16 @@ struct AParams {
   int n_inline;                       // > 0: use bars_inline
   const Tile* tiles;
   int n_tiles;
-  int nc_max;
   int per_max;             // adj_state_doubles of the largest member
   double dt;
   uint32_t* status;
-  double* scratch;
-  size_t scratch_per_cta;  // doubles
+  double* scratch;         // 2 NF doubles of every thread
   GitmVertParams prm;
-  // states saved by the SAVE step kernel (gitm_vert_plan_advance_saving),
-  // state s of global column c at saved[(s * saved_ncols + c) * per_max];
-  // NULL: the kernel recomputes them
+  // states saved by the saving step kernel, state s of the plan's column c at
+  // saved[(s * saved_ncols + c - saved_c0) * per_max]
   const double* saved;
   int64_t saved_ncols;
+  int64_t saved_c0;
 };
 
 // ---------------------------------------------------------------- helpers
@@ -652,18 +649,31 @@ __device__ inline double cell_adjoint_species(const ColCtx& c, const ColAdj& a, 
     const double Ls = c.x(F_LNS + s, i), Ws = c.x(F_W + s, i);
     const double divw = gW + 2 * Ws * invr;
     const double nl = Ls - dt * (divw + Ws * gL) + dt * dL;
-    menl[s] = c_k.mass[s] * exp(nl);
-    sumrho = sumrho + menl[s];
+    menl[s] = nl;
     const double km = c_k.k_over_m[s];
     double w = Ws - dt * (Ws * gW - hz + T * gL * km + gT * km - grav) + dt * dW - Ws * itau;
     w = w + cor;
     w = w - dt * (prm.thermal_diff_coef[s] * km) * gT;
     wv[s] = w;
   }
-  double ns[NS];
+  double ns[NS], ir;
+  {
+    double e[NS];
+    exp_n(menl, e);
 #pragma unroll
-  for (int s = 0; s < NS; ++s) ns[s] = exp(c.x(F_LNS + s, i));
-  const double ir = exp(-LR);
+    for (int s = 0; s < NS; ++s) {
+      menl[s] = c_k.mass[s] * e[s];
+      sumrho = sumrho + menl[s];
+    }
+    double l7[NS + 1], e7[NS + 1];
+#pragma unroll
+    for (int s = 0; s < NS; ++s) l7[s] = c.x(F_LNS + s, i);
+    l7[NS] = -LR;
+    exp_n(l7, e7);
+#pragma unroll
+    for (int s = 0; s < NS; ++s) ns[s] = e7[s];
+    ir = e7[NS];
+  }
   // reverse of New LogRho = log(sumrho): the continuity adjoints, with
   // New LogNS's own adjoint
   double nlb[NS];
@@ -678,59 +688,35 @@ __device__ inline double cell_adjoint_species(const ColCtx& c, const ColAdj& a, 
   // New VU = sum_s w_s m_s ns_s / Rho; New VertVel = the clamped w
   const double kvu = kb(F_VU);
   if (prm.use_neutral_friction) {
-    double glc[NS], lu[NS][NS], vsol[NS], pw[NS];
+    // the friction solve (friction_solve): S v = M n w
+    double glc[NS], mn[NS], vsol[NS], pe[NS];
     grad_log_cons(c, i, glc);
-    const double lt = log(T);
+    {
+      const double lt = log_sl(T);
+      double le[NS];
 #pragma unroll
-    for (int e = 0; e < NS; ++e) pw[e] = exp(c_k.one_minus_e[e] * lt);
-#pragma unroll
-    for (int r = 0; r < NS; ++r) {
-      double rs = 0.0;
-#pragma unroll
-      for (int q = 0; q < NS; ++q) {
-        if (q == r) continue;
-        const double cij = c_k.kc[r][q] * ns[q] * pw[exp_index(r, q)];
-        lu[r][q] = -dt * cij;
-        rs = rs + cij;
-      }
-      lu[r][r] = 1.0 + dt * rs;
-    }
-    // LU without pivoting: multipliers below the diagonal, pivot
-    // reciprocals on it (as friction_solve)
-#pragma unroll
-    for (int p = 0; p < NS; ++p) {
-      const double ip = rcp_nr(lu[p][p]);
-      lu[p][p] = ip;
-#pragma unroll
-      for (int r = p + 1; r < NS; ++r) {
-        const double l = lu[r][p] * ip;
-        lu[r][p] = l;
-#pragma unroll
-        for (int q = p + 1; q < NS; ++q) lu[r][q] -= l * lu[p][q];
-      }
+      for (int e = 0; e < NS; ++e) le[e] = c_k.one_minus_e[e] * lt;
+      exp_n(le, pe);
     }
 #pragma unroll
-    for (int r = 0; r < NS; ++r) {
-      double sum = wv[r];
+    for (int e = 0; e < NS; ++e) pe[e] = (dt * c_k.kpair[e]) * pe[e];
 #pragma unroll
-      for (int q = 0; q < r; ++q) sum -= lu[r][q] * vsol[q];
-      vsol[r] = sum;
+    for (int s = 0; s < NS; ++s) {
+      mn[s] = c_k.mass[s] * ns[s];
+      vsol[s] = mn[s] * wv[s];
     }
-#pragma unroll
-    for (int r = NS - 1; r >= 0; --r) {
-      double sum = vsol[r];
-#pragma unroll
-      for (int q = r + 1; q < NS; ++q) sum -= lu[r][q] * vsol[q];
-      vsol[r] = sum * lu[r][r];
-    }
+    FrictionLdl ldl;
+    ldl.factor(ns, mn, pe);
+    ldl.eliminate(vsol);
+    ldl.back(vsol);
     // clamp, bulk wind and their reverse
     double vb[NS];
 #pragma unroll
     for (int s = 0; s < NS; ++s) {
       const double v = vsol[s] + (-eddy * glc[s]);
       const bool inside = !(v < -prm.max_vertical_velocity) && !(v > prm.max_vertical_velocity);
-      double wc = fmax(-prm.max_vertical_velocity, v);
-      wc = fmin(prm.max_vertical_velocity, wc);
+      double wc = (v > -prm.max_vertical_velocity) ? v : -prm.max_vertical_velocity;
+      wc = (wc < prm.max_vertical_velocity) ? wc : prm.max_vertical_velocity;
       const double m = c_k.mass[s];
       const double wcb = kvu * (m * ns[s] * ir) + kb(F_W + s);
       nsb[s] = kvu * wc * m * ir;
@@ -756,46 +742,36 @@ __device__ inline double cell_adjoint_species(const ColCtx& c, const ColAdj& a, 
       a.gu[NS * a.nA + i - 1] = ul;
       LRb += lrb;
     }
-    // wb = M^-T vb with M = L U: U^T z = vb, then L^T wb = z
+    // (I + dt C) = (M n)^-1 S, so its transpose's solve is wb = M n y with S y = vb
 #pragma unroll
-    for (int r = 0; r < NS; ++r) {
-      double sum = vb[r];
-#pragma unroll
-      for (int q = 0; q < r; ++q) sum -= lu[q][r] * wb[q];
-      wb[r] = sum * lu[r][r];
-    }
-#pragma unroll
-    for (int r = NS - 1; r >= 0; --r) {
-      double sum = wb[r];
-#pragma unroll
-      for (int q = r + 1; q < NS; ++q) sum -= lu[q][r] * wb[q];
-      wb[r] = sum;
-    }
-    // M_rq = -dt C_rq (q != r), M_rr = 1 + dt sum_q C_rq:  Cb_rq = dt wb_r (vsol_q - vsol_r)
-    double pwb[NS];
-#pragma unroll
-    for (int e = 0; e < NS; ++e) pwb[e] = 0.0;
-#pragma unroll
-    for (int r = 0; r < NS; ++r)
-#pragma unroll
-      for (int q = 0; q < NS; ++q) {
-        if (q == r) continue;
-        const double cb = dt * wb[r] * (vsol[q] - vsol[r]);
-        const double k = c_k.kc[r][q];
-        nsb[q] += cb * k * pw[exp_index(r, q)];
-        pwb[exp_index(r, q)] += cb * k * ns[q];
-      }
+    for (int s = 0; s < NS; ++s) wb[s] = vb[s];
+    ldl.forward(wb);
+    ldl.back(wb);
+    // each pair (r, q) through its coefficient P = dt kpair T^(1-e), with y:
+    // n_q takes P n_r y_r (v_q - v_r), n_r takes P n_q y_q (v_r - v_q), and log T
+    // (1 - e) n_r n_q of both
     double ltb = 0.0;
 #pragma unroll
-    for (int e = 0; e < NS; ++e) ltb += pwb[e] * pw[e] * c_k.one_minus_e[e];
+    for (int r = 1; r < NS; ++r)
+#pragma unroll
+      for (int q = 0; q < r; ++q) {
+        const double P = pe[exp_index(r, q)];
+        const double t = P * (vsol[q] - vsol[r]);
+        const double ar = wb[r] * t, aq = -wb[q] * t;
+        nsb[q] = fma(ns[r], ar, nsb[q]);
+        nsb[r] = fma(ns[q], aq, nsb[r]);
+        ltb = fma(c_k.one_minus_e[exp_index(r, q)] * (ns[r] * ns[q]), ar + aq, ltb);
+      }
+#pragma unroll
+    for (int s = 0; s < NS; ++s) wb[s] *= mn[s];
     Tb += ltb / T;
   } else {
 #pragma unroll
     for (int s = 0; s < NS; ++s) {
       const double v = wv[s];
       const bool inside = !(v < -prm.max_vertical_velocity) && !(v > prm.max_vertical_velocity);
-      double wc = fmax(-prm.max_vertical_velocity, v);
-      wc = fmin(prm.max_vertical_velocity, wc);
+      double wc = (v > -prm.max_vertical_velocity) ? v : -prm.max_vertical_velocity;
+      wc = (wc < prm.max_vertical_velocity) ? wc : prm.max_vertical_velocity;
       const double m = c_k.mass[s];
       const double wcb = kvu * (m * ns[s] * ir) + kb(F_W + s);
       nsb[s] = kvu * wc * m * ir;
@@ -1058,9 +1034,8 @@ __global__ void __launch_bounds__(NT, 1) vert_adjoint_kernel(const AParams kp) {
   constexpr int nw = NT / 32;
   const GitmVertParams& prm = kp.prm;
   const double dt = kp.dt;
-  double* cta = kp.scratch + size_t(blockIdx.x) * kp.scratch_per_cta;
-  double* acc = cta + size_t(ADJ_NSTATE) * kp.nc_max * kp.per_max + tid;  // [NF] stride NT
-  double* kbs = acc + size_t(NF) * NT;                                     // [NF] stride NT
+  double* acc = kp.scratch + size_t(blockIdx.x) * (2 * NF * NT) + tid;  // [NF] stride NT
+  double* kbs = acc + size_t(NF) * NT;                                   // [NF] stride NT
 
   for (int tix = blockIdx.x; tix < kp.n_tiles; tix += gridDim.x) {
     const Tile tile = kp.tiles[tix];
@@ -1086,7 +1061,6 @@ __global__ void __launch_bounds__(NT, 1) vert_adjoint_kernel(const AParams kp) {
     const unsigned imask = __ballot_sync(0xffffffffu, item);
     const int nbl = (my_i == 1) ? NB_GHOST : (lane == 0) ? NB_WARP : NB_LANE;
     const int nbr = (my_i == nA) ? NB_GHOST : (lane == 31) ? NB_WARP : NB_LANE;
-    int cur = 0;
 
     auto ctx = [&](int cl) {
       ColCtx c;
@@ -1095,8 +1069,8 @@ __global__ void __launch_bounds__(NT, 1) vert_adjoint_kernel(const AParams kp) {
       c.gridc = M.gridc;
       c.gcols = M.gcols;
       c.gc = (M.gcols == 1) ? 0 : int(tile.c0 + cl);
-      c.xo = cur ? L.X1 : L.X0;
-      c.xpo = cur ? L.XP1 : L.XP0;
+      c.xo = L.X0;
+      c.xpo = L.XP0;
       return c;
     };
     auto adj = [&](int cl) {
@@ -1124,18 +1098,8 @@ __global__ void __launch_bounds__(NT, 1) vert_adjoint_kernel(const AParams kp) {
       return a;
     };
     auto gidx = [&](int f, int g, int cl) -> int64_t { return (int64_t(f) * G + g) * ncols + tile.c0 + cl; };
-    auto state = [&](int s, int cl) -> double* {
-      if (kp.saved)
-        return const_cast<double*>(kp.saved) +
-               (int64_t(s) * kp.saved_ncols + M.col_offset + tile.c0 + cl) * kp.per_max;
-      return cta + (size_t(s) * kp.nc_max + cl) * kp.per_max;
-    };
-    auto save = [&](int s, int off) {
-      for (int cl = 0; cl < nc; ++cl) {
-        const double* src = sm + size_t(A.stride) * cl + off;
-        double* dst = state(s, cl);
-        for (int r = tid; r < per; r += NT) dst[r] = src[r];
-      }
+    auto state = [&](int s, int cl) -> const double* {
+      return kp.saved + (int64_t(s) * kp.saved_ncols + M.col_offset + tile.c0 + cl - kp.saved_c0) * kp.per_max;
     };
     // (the caller's barrier publishes the copies)
     auto load = [&](int s, int off) {
@@ -1156,28 +1120,15 @@ __global__ void __launch_bounds__(NT, 1) vert_adjoint_kernel(const AParams kp) {
         }
       }
     };
-    auto boundaries = [&]() {
-      if (2 * nc <= nw) {
-        if (wid < 2 * nc) bc_column(ctx(wid >> 1), prm, lane, &sst[wid >> 1], 1 + (wid & 1));
-      } else {
-        for (int cl = wid; cl < nc; cl += nw) bc_column(ctx(cl), prm, lane, &sst[cl], 3);
-      }
-    };
     // bc^T of every column on the state in X0 with the pre-boundary ghost
     // values of saved state s_pre; a warp per column, or per column half
     // when the halves' interior cells are disjoint
     auto boundaries_adjoint = [&](int s_pre) {
-      if (2 * nc <= nw && nA >= 10) {
-        if (wid < 2 * nc) {
-          const int cl = wid >> 1;
-          const double* pre = state(s_pre, cl);
-          bc_column_adjoint(ctx(cl), adj(cl), pre, pre + NF * G, prm, lane, &sst[cl], 1 + (wid & 1));
-        }
-      } else {
-        for (int cl = wid; cl < nc; cl += nw) {
-          const double* pre = state(s_pre, cl);
-          bc_column_adjoint(ctx(cl), adj(cl), pre, pre + NF * G, prm, lane, &sst[cl], 3);
-        }
+      const int halves = (2 * nc <= nw && nA >= 10) ? 1 : 0;
+      for (int t = wid; t < (nc << halves); t += nw) {
+        const int cl = t >> halves;
+        const double* pre = state(s_pre, cl);
+        bc_column_adjoint(ctx(cl), adj(cl), pre, pre + NF * G, prm, lane, &sst[cl], halves ? 1 + (t & 1) : 3);
       }
     };
 
@@ -1188,7 +1139,8 @@ __global__ void __launch_bounds__(NT, 1) vert_adjoint_kernel(const AParams kp) {
     __syncthreads();
 
     // ------------------------------------------------------------ gather
-    // as the forward kernel's load (IO = 0), into X0
+    // the column scalars and coefficients, as the forward kernel's load; the
+    // state itself comes from the saved stage states
     if (tid < nc) {
       ColCtx c = ctx(tid);
       const int64_t cc = tile.c0 + tid;
@@ -1258,25 +1210,6 @@ __global__ void __launch_bounds__(NT, 1) vert_adjoint_kernel(const AParams kp) {
       c.gm(i) = gamma;
       if (i == -1) c.sc(SC_MMM_M1) = mmm;
       if (i == 0) c.sc(SC_MMM_0) = mmm;
-      // with saved stage states the state itself comes from them
-      if (kp.saved) continue;
-#pragma unroll
-      for (int s = 0; s < NS; ++s) {
-        c.x(F_LNS + s, i) = log(nd[s]);
-        c.x(F_W + s, i) = ww[s];
-      }
-      c.x(F_T, i) = temperature * tu;
-      c.x(F_VE, i) = b.velocity[gidx(0, g, cl)];
-      c.x(F_VN, i) = b.velocity[gidx(1, g, cl)];
-      c.x(F_VU, i) = b.velocity[gidx(2, g, cl)];
-      c.x(F_LRHO, i) = log(b.rho[gidx(0, g, cl)]);
-      const bool pc = in_pcells(i, nA);
-#pragma unroll
-      for (int s = 0; s < NI; ++s) {
-        if (s >= NADV && !pc) continue;
-        const double v = b.idensity_s[gidx(s, g, cl)];
-        c.ion(s, i) = prm.use_improved_ion_advection ? v : log(v);
-      }
     }
     __syncthreads();  // @phase 0
     double eddy = 0.0, ivup = 0.0;
@@ -1284,68 +1217,8 @@ __global__ void __launch_bounds__(NT, 1) vert_adjoint_kernel(const AParams kp) {
       eddy = b.eddy[gidx(0, my_i + 1, my_cl)];
       ivup = b.ivel_up[gidx(0, my_i + 1, my_cl)];
     }
-    if (kp.saved) {
-      // the step's states come from the saving forward: X4 into X0
-      load(5, L.X0);
-      __syncthreads();
-    } else {
-      save(0, L.X0);
-      __syncthreads();  // @phase 0
-      boundaries();
-      __syncthreads();  // @phase 1
-      save(1, L.X0);
-      // Orig := X0
-      for (int cl = 0; cl < nc; ++cl) {
-        double* col = sm + size_t(A.stride) * cl;
-        for (int r = tid; r < per; r += NT) col[L.O + r] = col[L.X0 + r];
-      }
-      __syncthreads();  // @phase 1
-
-      // ------------------------------------------------------------ forward
-      for (int k = 0; k < 4; ++k) {
-        for (int j = tid; j < nc * (nA + 2); j += NT) {
-          const int cl = j / (nA + 2), i = j - cl * (nA + 2);
-          rusanov_slopes_cell(ctx(cl), i, prm.beta_limiter);
-        }
-        __syncthreads();  // @phase 2
-        const int nxo = cur ? L.X0 : L.X1;
-        if (item) {
-          ColCtx c = ctx(my_cl);
-          const int i = my_i;
-          double* xn = c.col + nxo + 1;
-          auto emit = [&](int f, double kval) {
-            double& ag = acc[size_t(f) * NT];
-            const double a = (k == 0) ? kval : (k < 3) ? ag + 2.0 * kval : ag + kval;
-            ag = a;
-            const double o = c.o(f, i);
-            xn[f * G + i] = (k < 2) ? o + 0.5 * kval : (k == 2) ? o + kval : o + (1.0 / 6.0) * a;
-          };
-          rusanov_cell(c, i, prm, dt, eddy, ivup, 1.0 / prm.vert_tau, emit);
-        }
-        {
-          const int pr = NF * 4 + NPAS * NPC;
-          const int nxpo = cur ? L.XP0 : L.XP1;
-          for (int w = tid; w < nc * pr; w += NT) {
-            const int cl = w / pr, r = w - cl * pr;
-            double* col = sm + size_t(A.stride) * cl;
-            if (r < NF * 4) {
-              const int f = r >> 2, u = r & 3;
-              const int g = (u < 2) ? u : nA + u;
-              col[nxo + f * G + g] = col[L.O + f * G + g];
-            } else {
-              col[nxpo + r - NF * 4] = col[L.OP + r - NF * 4];
-            }
-          }
-        }
-        cur ^= 1;
-        __syncthreads();  // @phase 3
-        boundaries();
-        __syncthreads();  // @phase 4
-        save(2 + k, cur ? L.X1 : L.X0);
-        __syncthreads();  // @phase 1
-      }
-    }
-    // cur == 0: X4 is in X0
+    load(5, L.X0);  // X4
+    __syncthreads();
 
     // ------------------------------------------------------------ reverse
     for (int cl = 0; cl < nc; ++cl) {
@@ -1419,94 +1292,89 @@ __global__ void __launch_bounds__(NT, 1) vert_adjoint_kernel(const AParams kp) {
       }
     }
     __syncthreads();  // @phase 5
-    boundaries_adjoint(1);  // X4's boundaries: pre-boundary ghosts are Orig's
     if (tid < nc && !sfrozen[tid] && b.heating && B.heating_scale) {
       const double* hv = sm + size_t(A.stride) * tid + A.GU;
       double sum = 0.0;
       for (int i = 0; i < nA; ++i) sum += hv[i];
       sm[size_t(A.stride) * tid + A.MMB + 2] += sum;
     }
-    __syncthreads();  // @phase 6
-    // combination^T of the final: X4pre = Orig + (K0 + 2K1 + 2K2 + K3) / 6
-    if (item) {
-      ColAdj a = adj(my_cl);
-#pragma unroll
-      for (int f = 0; f < NF; ++f) {
-        const double ab = (1.0 / 6.0) * a.x(f, my_i);
-        acc[size_t(f) * NT] = ab;
-        kbs[size_t(f) * NT] = ab;  // K3bar = Abar
-      }
-    }
-    __syncthreads();  // @phase 7
-    fold(L.O, L.X1);
-    __syncthreads();  // @phase 7
-
-    const double wk[4] = {1.0, 2.0, 2.0, 1.0};
-    const double ck[3] = {0.5, 0.5, 1.0};
     double eddy_bar = 0.0;  // the four stages' KappaEddyDiffusion adjoints of this thread's cell
-    for (int k = 3; k >= 0; --k) {
-      load(1 + k, L.X0);
-      for (int cl = 0; cl < nc; ++cl) {
-        double* db = sm + size_t(A.stride) * cl + A.DB;
-        for (int r = tid; r < NSTENCIL * (nA + 2); r += NT) db[r] = 0.0;
-      }
-      for (int r = tid; r < ADJ_EDGE_DOUBLES; r += NT) eb[r] = 0.0;
-      __syncthreads();  // @phase 8
-      for (int j = tid; j < nc * (nA + 2); j += NT) {
-        const int cl = j / (nA + 2), i = j - cl * (nA + 2);
-        slopes_with_branches(ctx(cl), adj(cl), i, prm.beta_limiter);
-      }
-      __syncthreads();  // @phase 8
-      if (item) {
-        ColCtx c = ctx(my_cl);
-        ColAdj a = adj(my_cl);
-        eddy_bar += cell_adjoint_species(c, a, my_i, prm, dt, eddy, kbs, NT);
-        cell_adjoint_rest(c, a, my_i, dt, ivup, kbs, NT);
-        // K = New - state: the state's own -K
-#pragma unroll
-        for (int f = 0; f < NF; ++f) a.own(f, my_i, -kbs[size_t(f) * NT]);
-      }
-      __syncthreads();  // @phase 9
-      // GradLogConS's shares of the neighbouring cells and the sweeps'
-      // shares that crossed a warp boundary, one thread per cell
-      for (int w = tid; w < nc * G; w += NT) {
-        const int cl = w / G, m = w - cl * G - 1;
-        cell_gather(ctx(cl), adj(cl), m, cl * nA, nitems);
-      }
-      __syncthreads();  // @phase 9
-      {
-        // (column, field, run of cells) per thread
-        const int nseg = max(1, NT / (nc * NSTENCIL));
-        const int seg = (G + nseg - 1) / nseg;
-        for (int w = tid; w < nc * NSTENCIL * nseg; w += NT) {
-          const int sg = w % nseg, r = w / nseg, f = r % NSTENCIL, cl = r / NSTENCIL;
-          const int j0 = -1 + sg * seg, j1 = min(j0 + seg - 1, nA + 2);
-          if (j0 <= j1) slopes_adjoint_window(ctx(cl), adj(cl), f, j0, j1, prm.beta_limiter);
-        }
-      }
-      __syncthreads();  // @phase 10
-      if (k > 0) {
-        boundaries_adjoint(1);
-        __syncthreads();  // @phase 6
-        if (item) {
-          ColAdj a = adj(my_cl);
-#pragma unroll
-          for (int f = 0; f < NF; ++f)
-            kbs[size_t(f) * NT] = wk[k - 1] * acc[size_t(f) * NT] + ck[k - 1] * a.x(f, my_i);
-        }
-        __syncthreads();  // @phase 7
-        fold(L.O, L.X1);
-        __syncthreads();  // @phase 7
-      } else {
-        // X0 is also Orig
+    // the boundary pass of the final state, then stage k and the boundary
+    // pass of its state for k = 3 .. 0: one copy of each in the loop
+#pragma unroll 1
+    for (int k = 4;; --k) {
+      if (k < 4) {
+        load(1 + k, L.X0);
         for (int cl = 0; cl < nc; ++cl) {
-          double* col = sm + size_t(A.stride) * cl;
-          for (int r = tid; r < per; r += NT) col[L.X1 + r] += col[L.O + r];
+          double* db = sm + size_t(A.stride) * cl + A.DB;
+          for (int r = tid; r < NSTENCIL * (nA + 2); r += NT) db[r] = 0.0;
         }
-        __syncthreads();  // @phase 7
-        boundaries_adjoint(0);  // the first boundary pass: pre-boundary values are the gathered ones
-        __syncthreads();  // @phase 6
+        for (int r = tid; r < ADJ_EDGE_DOUBLES; r += NT) eb[r] = 0.0;
+        __syncthreads();  // @phase 8
+        for (int j = tid; j < nc * (nA + 2); j += NT) {
+          const int cl = j / (nA + 2), i = j - cl * (nA + 2);
+          slopes_with_branches(ctx(cl), adj(cl), i, prm.beta_limiter);
+        }
+        __syncthreads();  // @phase 8
+        if (item) {
+          ColCtx c = ctx(my_cl);
+          ColAdj a = adj(my_cl);
+          eddy_bar += cell_adjoint_species(c, a, my_i, prm, dt, eddy, kbs, NT);
+          cell_adjoint_rest(c, a, my_i, dt, ivup, kbs, NT);
+          // K = New - state: the state's own -K
+  #pragma unroll
+          for (int f = 0; f < NF; ++f) a.own(f, my_i, -kbs[size_t(f) * NT]);
+        }
+        __syncthreads();  // @phase 9
+        // GradLogConS's shares of the neighbouring cells and the sweeps'
+        // shares that crossed a warp boundary, one thread per cell
+        for (int w = tid; w < nc * G; w += NT) {
+          const int cl = w / G, m = w - cl * G - 1;
+          cell_gather(ctx(cl), adj(cl), m, cl * nA, nitems);
+        }
+        __syncthreads();  // @phase 9
+        {
+          // (column, field, run of cells) per thread
+          const int nseg = max(1, NT / (nc * NSTENCIL));
+          const int seg = (G + nseg - 1) / nseg;
+          for (int w = tid; w < nc * NSTENCIL * nseg; w += NT) {
+            const int sg = w % nseg, r = w / nseg, f = r % NSTENCIL, cl = r / NSTENCIL;
+            const int j0 = -1 + sg * seg, j1 = min(j0 + seg - 1, nA + 2);
+            if (j0 <= j1) slopes_adjoint_window(ctx(cl), adj(cl), f, j0, j1, prm.beta_limiter);
+          }
+        }
+        __syncthreads();  // @phase 10
+        if (k == 0) {
+          // X0 is also Orig
+          for (int cl = 0; cl < nc; ++cl) {
+            double* col = sm + size_t(A.stride) * cl;
+            for (int r = tid; r < per; r += NT) col[L.X1 + r] += col[L.O + r];
+          }
+          __syncthreads();  // @phase 7
+        }
       }
+      // pre-boundary ghosts: Orig's, the gathered ones for the first pass
+      boundaries_adjoint(k > 0 ? 1 : 0);
+      __syncthreads();  // @phase 6
+      if (k == 0) break;
+      if (item) {
+        // combination^T: X4pre = Orig + (K0 + 2 K1 + 2 K2 + K3) / 6, Xkpre = Orig + c K(k-1), c = 1/2, 1/2, 1
+        ColAdj a = adj(my_cl);
+        const double w = (k == 3 || k == 2) ? 2.0 : 1.0, cx = (k == 3) ? 1.0 : 0.5;
+#pragma unroll
+        for (int f = 0; f < NF; ++f) {
+          const double x = a.x(f, my_i);
+          double ab = (1.0 / 6.0) * x;
+          if (k == 4)
+            acc[size_t(f) * NT] = ab;
+          else
+            ab = w * acc[size_t(f) * NT] + cx * x;
+          kbs[size_t(f) * NT] = ab;
+        }
+      }
+      __syncthreads();  // @phase 7
+      fold(L.O, L.X1);
+      __syncthreads();  // @phase 7
     }
 
     if (item && B.eddy && !sfrozen[my_cl]) B.eddy[gidx(0, my_i + 1, my_cl)] += eddy_bar;
