@@ -22,9 +22,12 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 BUILD = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libgitmvert.so")
-SOURCES = ["gitm_vert.cu", "vert_adjoint.cu", "hz_kernel.cu"]
+SOURCES = ["gitm_vert.cu", "vert_adjoint.cu", "hz_kernel.cu", "vert_grid.cu"]
+# the grid coefficients round as the reference's, which uses no fused multiply-add
+EXTRA_FLAGS = {"vert_grid.cu": ["-fmad=false"]}
 DEPS = ["gitm_vert.cu", "vert_adjoint.cu", "hz_kernel.cu", "vert_instance.cu", "vert_instances.h", "vert_kernel.cuh",
-        "vert_ausm.cuh", "vert_adjoint.cuh", "vert_common.cuh", "vert_hz.cuh", "vert_math.cuh", "vert_tile.cu", "vert_tile.cuh"]
+        "vert_ausm.cuh", "vert_adjoint.cuh", "vert_common.cuh", "vert_hz.cuh", "vert_math.cuh", "vert_tile.cu", "vert_tile.cuh",
+        "vert_grid.cu", "vert_grid.cuh"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -81,7 +84,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
         return LIB
     os.makedirs(BUILD, exist_ok=True)
     extra = ["-Xptxas", "-v"] if verbose else []
-    jobs = [(os.path.join(CSRC, s), [], os.path.join(BUILD, s[:-3] + ".o")) for s in SOURCES]
+    jobs = [(os.path.join(CSRC, s), EXTRA_FLAGS.get(s, []), os.path.join(BUILD, s[:-3] + ".o")) for s in SOURCES]
     # the adjoint kernel for members of 50 altitudes, in a unit of its own
     jobs.append((os.path.join(CSRC, "vert_adjoint.cu"), ["-DGV_ADJ_NA=50"], os.path.join(BUILD, "vert_adjoint_n50.o")))
     jobs += [(os.path.join(CSRC, "vert_instance.cu"), flags, os.path.join(BUILD, f"step_{gid}.o"))

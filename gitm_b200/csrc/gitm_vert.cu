@@ -23,6 +23,7 @@
 #include "vert_adjoint.cuh"
 #include "vert_instances.h"
 #include "vert_hz.cuh"
+#include "vert_grid.cuh"
 
 using namespace gv;
 
@@ -155,88 +156,6 @@ static void fill_consts(Consts& k) {
       //      = 1e-2 k / (M_i D0_ij) * n_j * T^(1-e)   (calc_neutral_friction.f90:66-72)
       k.kc[i][j] = 1.0e-2 * KB / (mass[i] * (1.0e17 * d0[i][j]));
     }
-}
-
-// ------------------------------------------------------------------ grid
-// Grid coefficients of one column, in the reference's operation order:
-// dAlt_F / InvDAlt_F (advance_vertical.f90:149-151), the 5-point GradLogConS
-// mesh (vertical_solver_rusanov.f90:515-533) and the one-sided boundary
-// meshes (set_vertical_bcs.Earth.f90:279-297, 505-525).
-static size_t grid_rows(int G) { return size_t(NGC) * G + NBC + size_t(NGA) * G; }
-
-static void grid_coefs(int nA, const double* alt, const double* grav, const double* dalt_c,
-                       const double* inv_r, double* out /* [grid_rows(G)] */) {
-  const int G = nA + 4;
-  std::vector<double> dAF(G), IDF(G);
-  auto A = [&](int i) { return alt[i + 1]; };
-  for (int i = 0; i <= nA + 2; ++i) dAF[i + 1] = A(i) - A(i - 1);
-  dAF[0] = dAF[1];
-  for (int g = 0; g < G; ++g) IDF[g] = 1.0 / dAF[g];
-  auto F = [&](int i) { return dAF[i + 1]; };
-  std::fill(out, out + grid_rows(G), 0.0);
-  for (int g = 0; g < G; ++g) {
-    out[GC_DALTF * G + g] = dAF[g];
-    out[GC_H2 * G + g] = IDF[g] * 2.0;
-    out[GC_IDF * G + g] = IDF[g];
-    out[GC_IDC * G + g] = 1.0 / dalt_c[g];
-    out[GC_GRAV * G + g] = grav[g];
-    out[GC_INVR * G + g] = inv_r[g];
-    out[GC_R * G + g] = 1.0 / inv_r[g];
-    out[GC_ALT * G + g] = alt[g];
-  }
-  for (int i = 1; i <= nA; ++i) {
-    const double h1 = F(i - 1), h2 = F(i), h3 = F(i + 1), h4 = F(i + 2);
-    const double H2 = h2 + h1, H3 = h3 + h2 + h1, H4 = h4 + h3 + h2 + h1;
-    const double c0 = (h2 * h3 * (h3 + h4)) / (h1 * H2 * H3 * H4);
-    const double c1 = -1.0 * (H2 * h3 * (h3 + h4)) / (h1 * h2 * (h2 + h3) * (h2 + h3 + h4));
-    const double c3 = H2 * h2 * (h4 + h3) / (H3 * (h2 + h3) * h3 * h4);
-    const double c4 = -1.0 * H2 * h2 * h3 / (H4 * (h2 + h3 + h4) * (h3 + h4) * h4);
-    const double c2 = (h2 * h3 * (h3 + h4) + H2 * h3 * (h3 + h4) - H2 * h2 * (h3 + h4) - H2 * h2 * h3) /
-                      (H2 * h2 * h3 * (h3 + h4));
-    const double cs[5] = {c0, c1, c2, c3, c4};
-    for (int k = 0; k < 5; ++k) out[(GC_M0 + k) * G + i + 1] = cs[k];
-  }
-  double* bc = out + NGC * G;
-  for (int k = 0; k < 2; ++k) {  // lower: cells 0, -1
-    const int iAlt = -k;
-    const double h1 = F(iAlt + 2), h2 = F(iAlt + 3), h3 = F(iAlt + 4), h4 = F(iAlt + 5);
-    const double M1 = h1, M2 = h1 + h2, M3 = h1 + h2 + h3, M4 = h1 + h2 + h3 + h4;
-    bc[5 * k + 0] = -1.0 * (M2 * M3 * M4 + M1 * M3 * M4 + M1 * M2 * M4 + M1 * M2 * M3) / (M1 * M2 * M3 * M4);
-    bc[5 * k + 1] = 1.0 * (M2 * M3 * M4) / (h1 * h2 * (h2 + h3) * (h2 + h3 + h4));
-    bc[5 * k + 2] = -1.0 * (M1 * M3 * M4) / (M2 * h2 * h3 * (h3 + h4));
-    bc[5 * k + 3] = 1.0 * (M1 * M2 * M4) / (M3 * (h3 + h2) * h3 * h4);
-    bc[5 * k + 4] = -1.0 * (M1 * M2 * M3) / (M4 * (h2 + h3 + h4) * (h3 + h4) * h4);
-  }
-  for (int k = 0; k < 2; ++k) {  // upper: cells nA+1, nA+2
-    const int iAlt = nA + 1 + k;
-    const double h1 = F(iAlt - 1), h2 = F(iAlt - 2), h3 = F(iAlt - 3), h4 = F(iAlt - 4);
-    const double M1 = h1, M2 = h1 + h2, M3 = h1 + h2 + h3, M4 = h1 + h2 + h3 + h4;
-    bc[10 + 5 * k + 0] = 1.0 * (M2 * M3 * M4 + M1 * M3 * M4 + M1 * M2 * M4 + M1 * M2 * M3) / (M1 * M2 * M3 * M4);
-    bc[10 + 5 * k + 1] = -1.0 * (M2 * M3 * M4) / (h1 * h2 * (h2 + h3) * (h2 + h3 + h4));
-    bc[10 + 5 * k + 2] = 1.0 * (M1 * M3 * M4) / (M2 * h2 * h3 * (h3 + h4));
-    bc[10 + 5 * k + 3] = -1.0 * (M1 * M2 * M4) / (M3 * (h3 + h2) * h3 * h4);
-    bc[10 + 5 * k + 4] = 1.0 * (M1 * M2 * M3) / (M4 * (h2 + h3 + h4) * (h3 + h4) * h4);
-  }
-  // AUSM cell constants: the Kp / Ku altitude profiles
-  // (vertical_solver_ausm.f90:1314-1352), the spherical face areas and cell
-  // volume (:2029-2039) and the wind-diffusion factor (:944-946)
-  double* ga = out + NGC * G + NBC;
-  const double LogMaxKu = std::log(0.50), LogMinKu = std::log(0.25);
-  const double LogMaxKp = std::log(1.0e-09), LogMinKp = std::log(1.0e-19);
-  const double KpWidth = 15.0e+03, KpAltMidPoint = 160.0e+03;
-  auto R = [&](int i) { return 1.0 / inv_r[i + 1]; };
-  for (int g = 0; g < G; ++g) ga[GA_DALTC * G + g] = dalt_c[g];
-  for (int i = 1; i <= nA; ++i) {
-    const double LeftRadius = 0.5 * (R(i) + R(i - 1));
-    const double RightRadius = 0.5 * (R(i) + R(i + 1));
-    ga[GA_AP * G + i + 1] = RightRadius * RightRadius;
-    ga[GA_AM * G + i + 1] = LeftRadius * LeftRadius;
-    ga[GA_VOL * G + i + 1] = (1.0 / 3.0) * (std::pow(RightRadius, 3.0) - std::pow(LeftRadius, 3.0));
-    const double th = std::tanh((A(i) - KpAltMidPoint) / KpWidth);
-    ga[GA_KP * G + i + 1] = std::exp(LogMinKp + 0.5 * (LogMaxKp - LogMinKp) * (1.0 + th));
-    ga[GA_KU * G + i + 1] = std::exp(LogMinKu + 0.5 * (LogMaxKu - LogMinKu) * (1.0 + th));
-    ga[GA_DAMP * G + i + 1] = 0.35 * std::exp(-1.0 * (A(i) - A(0)) / (45.0e+03));
-  }
 }
 
 // ------------------------------------------------------------------ kernels
@@ -541,41 +460,41 @@ static bool is_device_ptr(const void* p) {
 static int plan_common(GitmVertPlan* P, const double* const* alt, const double* const* grav,
                        const double* const* dalt, const double* const* invr, const int* gpc) {
   GitmVertCtx* ctx = P->ctx;
-  // grid coefficients: copy each member's grid to the host, compute, upload
-  std::vector<size_t> goff(P->n_members);
+  // grid coefficients, formed on the device (vert_grid.cu); a member whose
+  // grid is in host memory has it copied behind the coefficients first
+  std::vector<size_t> goff(P->n_members), hoff(P->n_members, 0);
+  std::vector<double> host_grids;
   size_t gtotal = 0;
   for (int m = 0; m < P->n_members; ++m) {
     const GitmColumnBatch& b = P->host_members[m];
-    const int G = b.n_alts + 4;
     const int64_t gcols = gpc[m] ? b.n_cols : 1;
     goff[m] = gtotal;
-    gtotal += grid_rows(G) * gcols;
+    gtotal += grid_rows(b.n_alts + 4) * gcols;
   }
-  CUDA_TRY(ctx, cudaMalloc(&P->d_grid, gtotal * sizeof(double)));
+  for (int m = 0; m < P->n_members; ++m) {
+    const double* src[4] = {alt[m], grav[m], dalt[m], invr[m]};
+    bool device = true;
+    for (const double* p : src) device = device && is_device_ptr(p);
+    if (device) continue;
+    const int64_t per = int64_t(P->host_members[m].n_alts + 4) * (gpc[m] ? P->host_members[m].n_cols : 1);
+    hoff[m] = gtotal + host_grids.size();
+    for (const double* p : src) {
+      const size_t at = host_grids.size();
+      host_grids.resize(at + per);
+      CUDA_TRY(ctx, cudaMemcpy(host_grids.data() + at, p, per * sizeof(double), cudaMemcpyDefault));
+    }
+  }
+  CUDA_TRY(ctx, cudaMalloc(&P->d_grid, (gtotal + host_grids.size()) * sizeof(double)));
+  if (!host_grids.empty())
+    CUDA_TRY(ctx, cudaMemcpy(P->d_grid + gtotal, host_grids.data(), host_grids.size() * sizeof(double),
+                             cudaMemcpyHostToDevice));
   for (int m = 0; m < P->n_members; ++m) {
     const GitmColumnBatch& b = P->host_members[m];
-    const int nA = b.n_alts, G = nA + 4;
     const int64_t gcols = gpc[m] ? b.n_cols : 1;
-    const size_t per = size_t(G) * gcols;
-    std::vector<double> ha(per), hg(per), hd(per), hi(per);
-    CUDA_TRY(ctx, cudaMemcpy(ha.data(), alt[m], per * sizeof(double), cudaMemcpyDefault));
-    CUDA_TRY(ctx, cudaMemcpy(hg.data(), grav[m], per * sizeof(double), cudaMemcpyDefault));
-    CUDA_TRY(ctx, cudaMemcpy(hd.data(), dalt[m], per * sizeof(double), cudaMemcpyDefault));
-    CUDA_TRY(ctx, cudaMemcpy(hi.data(), invr[m], per * sizeof(double), cudaMemcpyDefault));
-    std::vector<double> colv(grid_rows(G)), out(grid_rows(G) * gcols);
-    std::vector<double> a1(G), g1(G), d1(G), i1(G);
-    for (int64_t gc = 0; gc < gcols; ++gc) {
-      for (int g = 0; g < G; ++g) {
-        a1[g] = ha[g * gcols + gc];
-        g1[g] = hg[g * gcols + gc];
-        d1[g] = hd[g * gcols + gc];
-        i1[g] = hi[g * gcols + gc];
-      }
-      grid_coefs(nA, a1.data(), g1.data(), d1.data(), i1.data(), colv.data());
-      for (size_t r = 0; r < grid_rows(G); ++r) out[r * gcols + gc] = colv[r];
-    }
-    CUDA_TRY(ctx, cudaMemcpy(P->d_grid + goff[m], out.data(), out.size() * sizeof(double),
-                             cudaMemcpyHostToDevice));
+    const int64_t per = int64_t(b.n_alts + 4) * gcols;
+    const double* h = hoff[m] ? P->d_grid + hoff[m] : nullptr;
+    CUDA_TRY(ctx, grid_launch(b.n_alts, gcols, h ? h : alt[m], h ? h + per : grav[m], h ? h + 2 * per : dalt[m],
+                              h ? h + 3 * per : invr[m], P->d_grid + goff[m], nullptr));
     P->dev_members_host[m].gridc = P->d_grid + goff[m];
     P->dev_members_host[m].gcols = int32_t(gcols);
   }
@@ -590,7 +509,10 @@ static int plan_common(GitmVertPlan* P, const double* const* alt, const double* 
   P->cfg.cols_per_cta = 0;
   P->cfg.steps_per_launch = 1;
   P->cfg.ctas_per_sm = 0;
-  return build_tiles(P);
+  const int rc = build_tiles(P);
+  // the plan's launches may go to any stream: its grid is ready from here on
+  CUDA_TRY(ctx, cudaStreamSynchronize(nullptr));
+  return rc;
 }
 
 static void plan_free(GitmVertPlan* P) {
@@ -1527,31 +1449,42 @@ __host__ __device__ inline int64_t fa_off(const GitmFArray& a, int lon, int lat,
 
 struct FMap {
   GitmFArray fa;  // Fortran side
-  int k;          // Fortran 4th index
+  GitmFArray fb;  // a second Fortran array that takes the same values (data NULL: none)
+  int k, kb;      // their Fortran 4th indices
   int64_t nat;    // offset of this field's first row in the native buffer
   int g_lo, g_hi; // cells copied (g = iAlt + 1); g_hi < g_lo: one value per column (iAlt = alt_fixed)
   int alt_fixed;
 };
 
-// dir 0: Fortran -> native; 1: native -> Fortran
-__global__ void fortran_copy_kernel(const FMap* maps, int nmaps, double* nat, int dir, int nLons, int nLats,
-                                    int bf, int64_t ncols, int G) {
+// dir 0: Fortran -> native; 1: native -> Fortran; either way the second
+// Fortran array takes the value too.  A thread per (column, part of the
+// cells): the column's indices are taken once, consecutive threads read
+// consecutive longitudes and write consecutive native columns.
+__global__ void __launch_bounds__(256) fortran_copy_kernel(const FMap* maps, double* nat, int dir, int nLons, int nLats,
+                                                           int bf, int ncols) {
   const FMap mp = maps[blockIdx.y];
-  const int64_t total = (mp.g_hi >= mp.g_lo) ? int64_t(mp.g_hi - mp.g_lo + 1) * ncols : ncols;
-  for (int64_t w = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; w < total; w += int64_t(gridDim.x) * blockDim.x) {
-    const int64_t c = w % ncols;
-    const int g = (mp.g_hi >= mp.g_lo) ? int(w / ncols) + mp.g_lo : -1;
-    const int lon = int(c % nLons) + 1;
-    const int lat = int((c / nLons) % nLats) + 1;
-    const int blk = int(c / (int64_t(nLons) * nLats)) + bf;
-    const int alt = (g >= 0) ? g - 1 : mp.alt_fixed;
-    double* f = mp.fa.data + fa_off(mp.fa, lon, lat, alt, mp.k, blk);
-    double* v = nat + mp.nat + ((g >= 0) ? int64_t(g) * ncols + c : c);
-    if (dir == 0) *v = *f;
-    else *f = *v;
+  const int c = blockIdx.x * 256 + threadIdx.x;
+  if (c >= ncols) return;
+  const int lon = c % nLons + 1, cl = c / nLons;
+  const int lat = cl % nLats + 1, blk = cl / nLats + bf;
+  const bool row = mp.g_hi >= mp.g_lo;
+  const int g0 = row ? mp.g_lo : 0, g1 = row ? mp.g_hi : 0;
+  double* f = mp.fa.data + fa_off(mp.fa, lon, lat, row ? -1 : mp.alt_fixed, mp.k, blk);  // cell g at f + g * stride[2]
+  double* f2 = mp.fb.data ? mp.fb.data + fa_off(mp.fb, lon, lat, -1, mp.kb, blk) : nullptr;
+  double* v = nat + mp.nat + c;
+  const int64_t sa = row ? mp.fa.stride[2] : 0, sb = mp.fb.stride[2];
+  const int step = gridDim.z;
+#pragma unroll 4
+  for (int g = g0 + blockIdx.z; g <= g1; g += step) {
+    double* fg = f + g * sa;
+    double* vg = v + int64_t(g) * ncols;
+    const double x = (dir == 0) ? *fg : *vg;
+    if (dir == 0)
+      *vg = x;
+    else
+      *fg = x;
+    if (f2) f2[g * sb] = x;
   }
-  (void)nmaps;
-  (void)G;
 }
 
 void host_copy(const FMap& mp, double* nat, int dir, int nLons, int nLats, int bf, int64_t ncols) {
@@ -1567,6 +1500,7 @@ void host_copy(const FMap& mp, double* nat, int dir, int nLons, int nLats, int b
     double* v = nat + mp.nat + ((g >= 0) ? int64_t(g) * ncols + c : c);
     if (dir == 0) *v = *f;
     else *f = *v;
+    if (mp.fb.data) mp.fb.data[fa_off(mp.fb, lon, lat, alt, mp.kb, blk)] = *v;
   }
 }
 
@@ -1579,6 +1513,8 @@ extern "C" int gitm_vert_advance_fortran(GitmVertCtx* ctx, const GitmFortranStat
   if (nLons <= 0 || nLats <= 0 || block_first < 1 || block_last < block_first || block_last > st->n_blocks)
     return set_err(ctx, GITM_ERR_ARG, "bad grid or block range");
   if (nA < 8 || nA > GITM_MAX_NALTS) return set_err(ctx, GITM_ERR_ARG, "n_alts out of range");
+  if (int64_t(nLons) * nLats * (block_last - block_first + 1) > int64_t(0x7fffff00))
+    return set_err(ctx, GITM_ERR_ARG, "too many columns");
   const GitmFArray* req[] = {&st->ndensity_s, &st->idensity_s, &st->rho, &st->temperature, &st->velocity,
                              &st->ivelocity, &st->vertical_velocity, &st->gamma, &st->mean_major_mass,
                              &st->temp_unit, &st->cmax, &st->kappa_eddy, &st->altitude, &st->gravity,
@@ -1596,11 +1532,15 @@ extern "C" int gitm_vert_advance_fortran(GitmVertCtx* ctx, const GitmFortranStat
                 o_cl = take(1), o_sz = take(1), o_ml = take(1), o_al = take(G), o_gr = take(G),
                 o_dz = take(G), o_ir = take(G);
   const int64_t n_nat = off;
-  std::vector<FMap> in, outm, sd_old, sd_new;
+  std::vector<FMap> in, outm;
+  GitmFArray none;
+  std::memset(&none, 0, sizeof none);
   auto add = [&](std::vector<FMap>& v, const GitmFArray& fa, int k, int64_t nat, int glo, int ghi, int altf = 0) {
     FMap m;
     m.fa = fa;
+    m.fb = none;
     m.k = k;
+    m.kb = 0;
     m.nat = nat;
     m.g_lo = glo;
     m.g_hi = ghi;
@@ -1636,14 +1576,21 @@ extern "C" int gitm_vert_advance_fortran(GitmVertCtx* ctx, const GitmFortranStat
   if (st->log_ns.data)
     for (int s = 0; s < NS; ++s) add(outm, st->log_ns, s + 1, o_lns + int64_t(s) * G * ncols, gl, gh);
   if (st->ndensity.data) add(outm, st->ndensity, 1, o_n, gl, gh);
-  // SpeciesDensity(Old)(:,:,:,1:nSpeciesTotal) = NDensityS; (nSpeciesTotal+1:) = IDensityS(1:nIons-1)
+  // SpeciesDensity(Old)(:,:,:,1:nSpeciesTotal) = NDensityS; (nSpeciesTotal+1:) = IDensityS(1:nIons-1),
+  // before the step (Old) and after it: the copies' second arrays
   auto species_maps = [&](std::vector<FMap>& v, const GitmFArray& sd) {
     if (!sd.data) return;
-    for (int s = 0; s < NS; ++s) add(v, sd, s + 1, o_nd + int64_t(s) * G * ncols, gl, gh);
-    for (int s = 0; s < GITM_NIONS - 1; ++s) add(v, sd, 11 + s + 1, o_id + int64_t(s) * G * ncols, gl, gh);
+    for (int s = 0; s < NS; ++s) {
+      v[s].fb = sd;
+      v[s].kb = s + 1;
+    }
+    for (int s = 0; s < GITM_NIONS - 1; ++s) {
+      v[NS + s].fb = sd;
+      v[NS + s].kb = 11 + s + 1;
+    }
   };
-  species_maps(sd_old, st->species_density_old);
-  species_maps(sd_new, st->species_density);
+  species_maps(in, st->species_density_old);
+  species_maps(outm, st->species_density);
 
   GitmVertParams saved = ctx->params;
   ctx->params.compute_coefficients = 0;
@@ -1671,36 +1618,44 @@ extern "C" int gitm_vert_advance_fortran(GitmVertCtx* ctx, const GitmFortranStat
     b.mlat = base + o_ml; b.altitude = base + o_al; b.gravity = base + o_gr; b.dalt_c = base + o_dz;
     b.inv_r = base + o_ir;
   }
+  FMap* d_maps = nullptr;  // the copies in, then out
   auto run_maps = [&](const std::vector<FMap>& v, int dir) -> int {
     if (v.empty()) return GITM_OK;
     if (!on_device) {
       for (const FMap& m : v) host_copy(m, base, dir, nLons, nLats, block_first, ncols);
       return GITM_OK;
     }
-    FMap* dm = nullptr;
-    CUDA_TRY(ctx, cudaMalloc(&dm, v.size() * sizeof(FMap)));
-    cudaMemcpy(dm, v.data(), v.size() * sizeof(FMap), cudaMemcpyHostToDevice);
-    const int64_t work = int64_t(G) * ncols;
-    dim3 grid(unsigned(std::min<int64_t>((work + 255) / 256, 4096)), unsigned(v.size()));
-    fortran_copy_kernel<<<grid, 256>>>(dm, int(v.size()), base, dir, nLons, nLats, block_first, ncols, G);
-    cudaError_t e = cudaDeviceSynchronize();
-    cudaFree(dm);
+    // cells in up to 8 parts, so that small calls fill the chip too
+    const dim3 grid(unsigned((ncols + 255) / 256), unsigned(v.size()), 8);
+    fortran_copy_kernel<<<grid, 256>>>(d_maps + (dir ? in.size() : 0), base, dir, nLons, nLats, block_first, int(ncols));
+    const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return set_err(ctx, GITM_ERR_CUDA, "fortran copy: %s", cudaGetErrorString(e));
     return GITM_OK;
   };
-  if (!rc) {
-    if (on_device) CUDA_TRY(ctx, cudaMemset(base, 0, size_t(n_nat) * sizeof(double)));
-    rc = run_maps(in, 0);
+  if (!rc && on_device) {
+    rc = [&]() -> int {
+      std::vector<FMap> all(in);
+      all.insert(all.end(), outm.begin(), outm.end());
+      CUDA_TRY(ctx, cudaMalloc(&d_maps, all.size() * sizeof(FMap)));
+      CUDA_TRY(ctx, cudaMemcpy(d_maps, all.data(), all.size() * sizeof(FMap), cudaMemcpyHostToDevice));
+      // cMax and the eddy coefficient have no outermost cells in the Fortran arrays
+      CUDA_TRY(ctx, cudaMemsetAsync(base + o_cm, 0, size_t(o_ed + G * ncols - o_cm) * sizeof(double), nullptr));
+      return GITM_OK;
+    }();
   }
-  if (!rc) rc = run_maps(sd_old, 1);  // SpeciesDensityOld = state before the step
+  if (!rc) rc = run_maps(in, 0);
   if (!rc) rc = on_device ? gitm_vert_advance_native(ctx, &b, 1, dt, 1)
                           : gitm_vert_advance_native_host(ctx, &b, 1, dt, 1);
   const bool column_err = (rc == GITM_ERR_COLUMN);
   if (!rc || column_err) {
     int rc2 = run_maps(outm, 1);
-    if (!rc2) rc2 = run_maps(sd_new, 1);
+    if (!rc2 && on_device) {
+      const cudaError_t e = cudaDeviceSynchronize();
+      if (e != cudaSuccess) rc2 = set_err(ctx, GITM_ERR_CUDA, "fortran copy: %s", cudaGetErrorString(e));
+    }
     if (rc2) rc = rc2;
   }
+  cudaFree(d_maps);
   ctx->params = saved;
   return rc;
 }

@@ -1,0 +1,22 @@
+// vert_grid.cuh -- host-side entry of the grid-coefficient kernel
+// (vert_grid.cu, its own translation unit).
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <cstddef>
+#include <cstdint>
+
+#include "vert_common.cuh"
+
+namespace gv {
+
+// Rows of one grid column's coefficients: [NGC][G], the boundary meshes, [NGA][G].
+__host__ __device__ inline size_t grid_rows(int G) { return size_t(NGC) * G + NBC + size_t(NGA) * G; }
+
+// Forms the coefficients of gcols grid columns (device arrays [G][gcols])
+// into out [grid_rows(G)][gcols].
+cudaError_t grid_launch(int nAlts, int64_t gcols, const double* alt, const double* grav, const double* dalt_c,
+                        const double* inv_r, double* out, cudaStream_t stream);
+
+}  // namespace gv
