@@ -5,18 +5,26 @@
 // Temperature, Velocity, the six NDensityS and VerticalVelocity, the advected
 // IDensityS: 19 fields) and its grid metrics are loaded with their two ghost
 // rings from GITM's own Fortran-layout arrays (a plane of one field is
-// contiguous there, longitude fastest) into shared memory; one thread per
-// interior cell runs the four RK stages of :168-345, each stage the whole
-// horizontal_solver (:535-818) at the thread's cell: for every field the
-// limited slopes of calc_facevalues_lons / _lats (:928-1034) at the cell and
-// its two neighbours, the face values, the Rusanov gradient and diffusion
-// (calc_rusanov_lons / _lats, :821-922), then the cell's equations.  The
-// ghost rings keep their values through the stages, as in the reference.
+// contiguous there, longitude fastest) into shared memory.  Each of the four
+// RK stages of :168-345 is three phases:
+//   slopes    the limited slopes of calc_facevalues_lons / _lats (:928-1034),
+//             one per field, direction and cell, to shared memory
+//   cells     horizontal_solver (:535-818): the face values, the Rusanov
+//             gradient and diffusion (calc_rusanov_lons / _lats, :821-922) and
+//             the equations, four threads per cell with five fields each
+//   update    Orig + c K, each thread its own fields
+// The ghost rings keep their values through the stages, as in the reference.
 // The store phase writes the interior cells back with the stores of
 // :346-421 and, with UseImprovedIonAdvection, the parallel ion-velocity
 // divergence of :423-517 (UAM_Gradient, gradient.f90:4-104) at the cell,
 // which reads only IVelocityPar and the grid; the CTA of the first and last
 // altitude also rewrite the electron sum of the ghost planes.
+//
+// What bounds it is the FP64 pipe and the latency of its chains.  With one
+// thread per cell and every slope formed by each of the three cells that read
+// it (486 per field of a 9 x 9 plane instead of 198), 12 warps ran per SM at
+// 168 registers, spilling, and a 2 degree globe (10,000 planes of 9 x 9) took
+// 3.11 ms; with the slopes shared and five fields per thread 1.31 ms.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -33,291 +41,360 @@ constexpr int HZ_NSW = 5 + 2 * NS + NADV;  // swept fields
 constexpr int NI_ALL = GITM_NIONS - 1;     // ions without the electrons
 constexpr int HF_R = 0, HF_T = 1, HF_V = 2, HF_N = 5, HF_W = 5 + NS, HF_I = 5 + 2 * NS;
 constexpr int HZ_NGP = 6;   // metric planes with ghost rings: IFB, DFB lon; IFB, DFB lat; cMax E, N
-constexpr int HZ_NGC = 7;   // metric values at interior cells: InvD*Dist_GB lon, lat; Gamma; InvR; R; IVel E, N
+constexpr int HZ_NLD = HZ_NSW + 4;  // planes loaded whole: the fields and the four metrics
+constexpr int HZ_PER = 5;   // fields of a thread
+constexpr int HZ_GRP = 4;   // threads of a cell: fields 5 g .. 5 g + 4
 constexpr double F1 = 0.6250000;  // Factor1, advance_horizontal.f90:939
 constexpr double F2 = 0.0416667;  // Factor2, advance_horizontal.f90:940
+static_assert(HZ_PER * HZ_GRP >= HZ_NSW && HF_N == HZ_PER, "the groups' fields");
 
-// Shared-memory plan of one plane: P cells with ghosts, C interior cells.
+// Shared-memory plan of one plane (doubles).  Rows of NIp cells and of NLp
+// longitude slopes are odd, so lanes on neighbouring rows do not collide
+// (padding rows and planes to be free of all collisions gained nothing).  P:
+// cells of a plane with ghosts, C: interior cells, per: slopes of a field
+// (lines along longitude, then along latitude, longitude fastest).
+// batch: the fields whose slopes are held at once, a multiple of HZ_PER (all
+// of them for every ordinary block; thin blocks of 2 x 128 cells take fewer).
+// keep: Orig and the RK accumulators of the cells are held here too, which
+// frees 20 registers of every thread, where there is room.
 struct HzLayout {
-  int P, C;
-  int S, K, G, GC, stride;
+  int NIp, P, C, NLp, NL, per;
+  int S, D, G, K, M, R, stride;  // M: Gamma, RadialDistance, IVelocity east and north of the cells;
+                                 // R: sin, cos and tan of the latitude of every interior row
 };
 
-__host__ __device__ inline HzLayout hz_layout(int nLons, int nLats) {
+__host__ __device__ inline HzLayout hz_layout(int nLons, int nLats, int batch, bool keep) {
   HzLayout L;
-  L.P = (nLons + 4) * (nLats + 4);
+  L.NIp = (nLons + 4) | 1;
+  L.NLp = (nLons + 2) | 1;
+  L.NL = L.NLp * nLats;
+  L.P = L.NIp * (nLats + 4);
+  L.per = L.NL + (nLats + 2) * nLons;
   L.C = nLons * nLats;
   int o = 0;
   L.S = o;  o += HZ_NSW * L.P;
-  L.K = o;  o += HZ_NSW * L.C;  // the stage's New - state of every field
+  L.D = o;  o += (batch < HZ_NSW ? batch : HZ_NSW) * L.per;
   L.G = o;  o += HZ_NGP * L.P;
-  L.GC = o; o += HZ_NGC * L.C;
+  L.K = o;  o += keep ? 2 * HZ_NSW * L.C : 0;
+  L.M = o;  o += keep ? 4 * L.C : 0;
+  L.R = o;  o += 3 * nLats;
   L.stride = o;
   return L;
 }
 
-// Limiter_mc (ModLimiter.f90:16-36) without branches: both candidates are
-// formed and the signs select one, so lanes of different cases do not split
-// the warp
+// ModLimiter.f90:16-36 without branches (limiter_mc of the vertical step).
 __device__ __forceinline__ double hz_limiter(double u, double d, double beta) {
-  const double bu = beta * u, bd = beta * d, av = (u + d) * 0.5;
-  const double lo = fmin(fmin(bu, bd), av), hi = fmax(fmax(bu, bd), av);
-  const bool pos = (u > 0.0) && (d > 0.0);
-  const bool neg = !(u > 0.0) && (d < 0.0);
-  return pos ? lo : (neg ? hi : 0.0);
+  const double au = fabs(u), ad = fabs(d);
+  const double t = beta * (au < ad ? au : ad);
+  const double s = (u + d) * 0.5, as = fabs(s);
+  const double m = t < as ? t : as;
+  const bool same = (__double2hiint(u) ^ __double2hiint(d)) >= 0;
+  const int hi = __double2hiint(m) | (__double2hiint(u) & int(0x80000000u));
+  return same ? __hiloint2double(hi, __double2loint(m)) : 0.0;
 }
 
-// The limited slope of line cell q (0 .. n+1) as calc_facevalues_lons /
-// _lats form it: the 4th-order differences, with the 2nd-order one on the
-// outer side of cells 0 and n+1.  V(q) = V[(q+1)*s], IF(q) = IF[(q+1)*s].
-__device__ __forceinline__ double hz_slope(const double* V, const double* IF, int s, int q, int n,
-                                           double beta) {
-  auto v = [&](int x) { return V[(x + 1) * s]; };
-  auto f = [&](int x) { return IF[(x + 1) * s]; };
-  // both forms in one expression: the 2nd-order side is h * (1 * (...) -
-  // 0 * (...)) with h = IF, exactly; the outer neighbours are clamped into
-  // the line (finite values the zero factor removes)
-  const bool eu = (q == n + 1), ed = (q == 0);
-  const double hu = eu ? f(q + 1) : f(q + 1) * 2, hd = ed ? f(q) : f(q) * 2;
-  const double au = eu ? 1.0 : F1, bu = eu ? 0.0 : F2, ad = ed ? 1.0 : F1, bd = ed ? 0.0 : F2;
-  const double up = hu * (au * (v(q + 1) - v(q)) - bu * (v(min(q + 2, n + 2)) - v(q - 1)));
-  const double dn = hd * (ad * (v(q) - v(q - 1)) - bd * (v(q + 1) - v(max(q - 2, -1))));
-  return hz_limiter(up, dn, beta);
+// The limited slopes of one line (calc_facevalues_lons / _lats): cells 0 ..
+// n+1 of values V and inverse face distances IF, both with stride s (index 0
+// = cell -1), to d with stride sd.  4th-order differences, with the 2nd-order
+// one on the outer side of cells 0 and n+1.  Along the line each value and
+// each difference is formed once: 3 shared-memory accesses and 11 FP64
+// instructions per slope (9 and 16 with a thread per slope).
+__device__ __forceinline__ void hz_slopes(const double* V, const double* IF, double* d, int s, int sd, int n,
+                                          double beta) {
+  double vm = V[0], v0 = V[s], vp = V[2 * s];  // cells -1, 0, 1
+  double dn = (v0 - vm) * IF[s];               // between cells -1 and 0: 2nd order
+#pragma unroll 4
+  for (int q = 0; q <= n; ++q) {
+    // between cells q and q+1
+    const double vq = V[(q + 3) * s];
+    const double up = (IF[(q + 2) * s] * 2) * (F1 * (vp - v0) - F2 * (vq - vm));
+    d[q * sd] = hz_limiter(up, dn, beta);
+    dn = up;
+    vm = v0;
+    v0 = vp;
+    vp = vq;
+  }
+  d[(n + 1) * sd] = hz_limiter((vp - v0) * IF[(n + 3) * s], dn, beta);
 }
 
-// calc_rusanov_lons / _lats at line cell p (1..n): the gradient and the
-// Rusanov diffusion from the face values of faces p and p+1.
-__device__ __forceinline__ void hz_line(const double* V, const double* IF, const double* DF, const double* CM,
-                                        int s, int p, int n, double invd, double beta, double& grad,
-                                        double& diff) {
-  const double sm = hz_slope(V, IF, s, p - 1, n, beta);
-  const double s0 = hz_slope(V, IF, s, p, n, beta);
-  const double sp = hz_slope(V, IF, s, p + 1, n, beta);
-  const double vm = V[p * s], v0 = V[(p + 1) * s], vp = V[(p + 2) * s];
-  const double d0 = DF[(p + 1) * s], d1 = DF[(p + 2) * s];
-  const double W0 = vm + 0.5 * sm * d0;  // VarLeft(p)
-  const double E0 = v0 - 0.5 * s0 * d0;  // VarRight(p)
-  const double W1 = v0 + 0.5 * s0 * d1;  // VarLeft(p+1)
-  const double E1 = vp - 0.5 * sp * d1;  // VarRight(p+1)
-  grad = 0.5 * (W1 + E1 - W0 - E0) * invd;
-  const double c0 = 0.5 * fmax(CM[p * s], CM[(p + 1) * s]) * (E0 - W0);
-  const double c1 = 0.5 * fmax(CM[(p + 1) * s], CM[(p + 2) * s]) * (E1 - W1);
-  diff = (c1 - c0) * invd;
-}
+// A cell's faces along one direction: halves of the face widths, the
+// dissipation coefficients times 1 / width, half of 1 / width.
+struct HzFaces {
+  double h0, h1, b0, b1, g;
+  // calc_rusanov_lons / _lats: gradient and diffusion from the slopes of the
+  // cell's line neighbours (sm, s0, sp) and their values
+  __device__ __forceinline__ void sweep(double vm, double v0, double vp, double sm, double s0, double sp, double& grad,
+                                        double& diff) const {
+    const double W0 = fma(sm, h0, vm), E0 = fma(-s0, h0, v0);
+    const double W1 = fma(s0, h1, v0), E1 = fma(-sp, h1, vp);
+    grad = (W1 + E1 - W0 - E0) * g;
+    diff = fma(b1, E1 - W1, -(b0 * (E0 - W0)));
+  }
+  __device__ __forceinline__ double grad(double vm, double v0, double vp, double sm, double s0, double sp) const {
+    return (fma(s0, h1, v0) + fma(-sp, h1, vp) - fma(sm, h0, vm) - fma(-s0, h0, v0)) * g;
+  }
+};
 
 struct HzArgs {
   GitmHzParams prm;
   GitmHzBlocks b;
   double dt;
   uint32_t* status;  // one word per block
+  int group;         // threads of a field group: the interior cells rounded up to whole warps
+  int batch;         // see hz_layout
+  unsigned magic;    // ceil(2^32 / lines of a field): w / lines = umulhi(w, magic) for w < 2^16
 };
 
-template <int NT, int MINB>
+// Threads: HZ_GRP groups of A.group (at most NT in all); thread q of a group
+// has interior cell q.
+template <int NT, int MINB, bool KEEP>
 __global__ void __launch_bounds__(NT, MINB) hz_step_kernel(const HzArgs A) {
   extern __shared__ double sm[];
   const GitmHzBlocks& B = A.b;
   const GitmHzParams& prm = A.prm;
   const int nl = B.n_lons, nt = B.n_lats, na = B.n_alts;
-  const int NI = nl + 4, NJ = nt + 4, NK = na + 4;
-  const int64_t P = int64_t(NI) * NJ, V = P * NK;
+  const int NG = nl + 4, NJ = nt + 4, NK = na + 4;
+  const int PG = NG * NJ;  // a plane of GITM's arrays
+  const int64_t V = int64_t(PG) * NK;
   const int k = blockIdx.x % na + 1;  // Fortran altitude of this plane
   const int b = blockIdx.x / na;
-  const int tid = threadIdx.x;
-  const HzLayout L = hz_layout(nl, nt);
+  const int tid = threadIdx.x, nthr = blockDim.x;
+  const HzLayout L = hz_layout(nl, nt, A.batch, KEEP);
+  const int NI = L.NIp, P = L.P;  // rows and planes in shared memory
   const double dt = A.dt;
   // first element of plane k of field f of a block array with nf fields
   auto plane = [&](const double* a, int f, int nf) -> const double* {
-    return a + ((int64_t(b) * nf + f) * NK + (k + 1)) * P;
+    return a + ((int64_t(b) * nf + f) * NK + (k + 1)) * PG;
   };
   auto lat1 = [&](const double* a, int j) { return a[int64_t(b) * NJ + (j + 1)]; };
 
   // ---------------------------------------------------------------- load
   double* S = sm + L.S;
-  double* Kc = sm + L.K;
+  double* D = sm + L.D;
   double* GP = sm + L.G;
-  double* GC = sm + L.GC;
   auto src_of = [&](int f) -> const double* {
     if (f == HF_R) return plane(B.rho, 0, 1);
     if (f == HF_T) return plane(B.temperature, 0, 1);
     if (f < HF_N) return plane(B.velocity, f - HF_V, 3);
     if (f < HF_W) return plane(B.ndensity_s, f - HF_N, GITM_NSPECIES_TOTAL);
     if (f < HF_I) return plane(B.vert_vel, f - HF_W, NS);
-    return plane(B.idensity_s, f - HF_I, GITM_NIONS);
+    if (f < HZ_NSW) return plane(B.idensity_s, f - HF_I, GITM_NIONS);
+    return plane(f == HZ_NSW ? B.inv_dlon_dist_fb : f == HZ_NSW + 1 ? B.dlon_dist_fb
+                 : f == HZ_NSW + 2 ? B.inv_dlat_dist_fb : B.dlat_dist_fb, 0, 1);
   };
-  for (int f = 0; f < HZ_NSW; ++f) {
+  // a field per warp and turn, straight into shared memory
+  for (int f = tid >> 5; f < HZ_NLD; f += nthr >> 5) {
     const double* src = src_of(f);
-    for (int c = tid; c < P; c += NT) S[f * P + c] = src[c];
+    double* dst = f < HZ_NSW ? S + f * P : GP + (f - HZ_NSW) * P;
+    for (int c = tid & 31; c < PG; c += 32) {
+      const int j = c / NG;
+      const uint32_t d = uint32_t(__cvta_generic_to_shared(dst + c + j * (NI - NG)));
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src + c) : "memory");
+    }
   }
   {
-    const double* gsrc[4] = {plane(B.inv_dlon_dist_fb, 0, 1), plane(B.dlon_dist_fb, 0, 1),
-                             plane(B.inv_dlat_dist_fb, 0, 1), plane(B.dlat_dist_fb, 0, 1)};
-    for (int g = 0; g < 4; ++g)
-      for (int c = tid; c < P; c += NT) GP[g * P + c] = gsrc[g][c];
     // cMax_GDB(0:nLons+1, 0:nLats+1, 0:nAlts+1, 3, nBlocks): east and north
-    // components of this altitude into planes with the outer ghost ring
-    // (never read) zeroed
-    const int ci2 = nl + 2, cj2 = nt + 2;
-    for (int d = 0; d < 2; ++d) {
-      const double* cm = B.cmax + (((int64_t(b) * 3 + d) * (na + 2) + k) * cj2) * ci2;
-      for (int c = tid; c < P; c += NT) {
-        const int i = c % NI - 1, j = c / NI - 1;  // Fortran indices
-        const bool in = (i >= 0 && i <= nl + 1 && j >= 0 && j <= nt + 1);
-        GP[(4 + d) * P + c] = in ? cm[j * ci2 + i] : 0.0;
-      }
+    // components of this altitude (the outer ghost ring is never read)
+    const int ci2 = nl + 2, n = ci2 * (nt + 2);
+    for (int w = tid; w < 2 * n; w += nthr) {
+      const int d = w >= n, c = w - d * n;
+      const int j = c / ci2, i = c - j * ci2;  // Fortran indices
+      GP[(4 + d) * P + (j + 1) * NI + i + 1] = B.cmax[((int64_t(b) * 3 + d) * (na + 2) + k) * n + c];
     }
   }
-  const bool cell = tid < L.C;
-  const int ci = cell ? tid % nl + 1 : 1, cj = cell ? tid / nl + 1 : 1;  // Fortran (iLon, iLat)
-  const int pc = (cj + 1) * NI + (ci + 1);                                // plane index of the cell
-  if (cell) {
-    GC[0 * L.C + tid] = plane(B.inv_dlon_dist_gb, 0, 1)[pc];
-    GC[1 * L.C + tid] = plane(B.inv_dlat_dist_gb, 0, 1)[pc];
-    GC[2 * L.C + tid] = plane(B.gamma, 0, 1)[pc];
-    GC[3 * L.C + tid] = plane(B.inv_radial_distance, 0, 1)[pc];
-    GC[4 * L.C + tid] = plane(B.radial_distance, 0, 1)[pc];
-    GC[5 * L.C + tid] = plane(B.ivelocity, 0, 3)[pc];
-    GC[6 * L.C + tid] = plane(B.ivelocity, 1, 3)[pc];
+  // what the equations read of other arrays at cell q: Gamma, RadialDistance, IVelocity east, north
+  auto other = [&](int m) -> const double* {
+    return m == 0 ? plane(B.gamma, 0, 1) : m == 1 ? plane(B.radial_distance, 0, 1) : plane(B.ivelocity, m - 2, 3);
+  };
+  if (KEEP) {
+    for (int w = tid; w < 4 * L.C; w += nthr) {
+      const int m = w / L.C, c = w - m * L.C;
+      const uint32_t d = uint32_t(__cvta_generic_to_shared(sm + L.M + w));
+      const double* src = other(m) + (c / nl + 2) * NG + (c % nl + 2);
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src) : "memory");
+    }
   }
-  // Orig (:181-186) stays in the input arrays: they are written only by the
-  // store phase, after the last stage
-
+  for (int j = tid; j < nt; j += nthr) {
+    sm[L.R + 3 * j] = sin(lat1(B.latitude, j + 1));
+    sm[L.R + 3 * j + 1] = lat1(B.cos_latitude, j + 1);
+    sm[L.R + 3 * j + 2] = lat1(B.tan_latitude, j + 1);
+  }
+  const int grp = tid / A.group, q = tid - grp * A.group;
+  const bool cell = q < L.C;
+  const int ci = cell ? q % nl + 1 : 1, cj = cell ? q / nl + 1 : 1;  // Fortran (iLon, iLat)
+  const int pc = (cj + 1) * NI + (ci + 1);  // the cell in a plane of shared memory
+  const int pg = (cj + 1) * NG + (ci + 1);  // and of GITM's arrays
   // per-cell constants of the equations (:680-686)
-  double SinLat = 0.0, CosLat = 0.0, TanLat = 0.0;
-  if (cell) {
-    SinLat = sin(lat1(B.latitude, cj));
-    CosLat = lat1(B.cos_latitude, cj);
-    TanLat = lat1(B.tan_latitude, cj);
-  }
-  const double CoriolisSin = SinLat * 2 * prm.omega_body;
-  const double CoriolisCos = CosLat * 2 * prm.omega_body;
-  const double CentrifugalParameter = (prm.omega_body * prm.omega_body) * CosLat * SinLat;
+  const double* row = sm + L.R + 3 * (cj - 1);
+  const double InvR = plane(B.inv_radial_distance, 0, 1)[pg];
   const double beta = prm.beta_limiter;
-  const double* IFlo = GP + 0 * P;
-  const double* DFlo = GP + 1 * P;
-  const double* IFla = GP + 2 * P;
-  const double* DFla = GP + 3 * P;
-  const double* CMe = GP + 4 * P;
-  const double* CMn = GP + 5 * P;
-
-  // the Rusanov gradient / diffusion of field f at the cell along lon, lat
-  auto lon_of = [&](int f, double& g, double& d) {
-    const int row = (cj + 1) * NI;
-    hz_line(S + f * P + row, IFlo + row, DFlo + row, CMe + row, 1, ci, nl, GC[0 * L.C + tid], beta, g, d);
-  };
-  auto lat_of = [&](int f, double& g, double& d) {
-    const int col = ci + 1;
-    hz_line(S + f * P + col, IFla + col, DFla + col, CMn + col, NI, cj, nt, GC[1 * L.C + tid], beta, g, d);
-  };
-
-  double acc[HZ_NSW];
+  const int f0 = grp * HZ_PER;  // this thread's fields
+  const int nf = min(HZ_PER, HZ_NSW - f0);
+  double orig_r[KEEP ? 1 : HZ_PER], acc_r[KEEP ? 1 : HZ_PER];
+  double* keep = sm + L.K + (cell ? f0 * L.C + q : 0);  // Orig of field f0 + j at keep[j C], its accumulator NSW C on
+  auto orig = [&](int j) -> double& { return KEEP ? keep[j * L.C] : orig_r[KEEP ? 0 : j]; };
+  auto acc = [&](int j) -> double& { return KEEP ? keep[(HZ_NSW + j) * L.C] : acc_r[KEEP ? 0 : j]; };
+  HzFaces lo, la;
+  {
+    const double il = plane(B.inv_dlon_dist_gb, 0, 1)[pg], it = plane(B.inv_dlat_dist_gb, 0, 1)[pg];
+    lo.g = 0.5 * il;
+    la.g = 0.5 * it;
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
+  {
+    const double* DFlo = GP + 1 * P;
+    const double* DFla = GP + 3 * P;
+    const double* CMe = GP + 4 * P;
+    const double* CMn = GP + 5 * P;
+    lo.h0 = 0.5 * DFlo[pc];
+    lo.h1 = 0.5 * DFlo[pc + 1];
+    lo.b0 = fmax(CMe[pc - 1], CMe[pc]) * lo.g;
+    lo.b1 = fmax(CMe[pc], CMe[pc + 1]) * lo.g;
+    la.h0 = 0.5 * DFla[pc];
+    la.h1 = 0.5 * DFla[pc + NI];
+    la.b0 = fmax(CMn[pc - NI], CMn[pc]) * la.g;
+    la.b1 = fmax(CMn[pc], CMn[pc + NI]) * la.g;
+  }
+#pragma unroll
+  for (int j = 0; j < HZ_PER; ++j)
+    if (cell && j < nf) orig(j) = S[(f0 + j) * P + pc];  // Orig (:181-186)
+
+  auto value = [&](int m) { return KEEP ? sm[L.M + m * L.C + q] : other(m)[pg]; };
+  // where the cell's slopes stand in a field's slope row
+  const int dl = (cj - 1) * L.NLp + ci, dt0 = L.NL + cj * nl + (ci - 1);
+  const int per = L.per, lines = nl + nt;
+  auto sweeps = [&](int f, int fb, double& gLo, double& gLa, double& dd) {
+    const double* v = S + f * P + pc;
+    const double* d = D + (f - fb) * per;
+    double dLo, dLa;
+    lo.sweep(v[-1], v[0], v[1], d[dl - 1], d[dl], d[dl + 1], gLo, dLo);
+    la.sweep(v[-NI], v[0], v[NI], d[dt0 - nl], d[dt0], d[dt0 + nl], gLa, dLa);
+    dd = dLo + dLa;
+  };
 
   // ---------------------------------------------------------------- RK4
+#pragma unroll 1
   for (int st = 0; st < 4; ++st) {
-    auto kv = [&](int f) -> double& { return Kc[f * L.C + tid]; };
-    if (cell) {
-      const double InvR = GC[3 * L.C + tid];
-      const double R = S[HF_R * P + pc], T = S[HF_T * P + pc];
-      const double VE = S[(HF_V + 0) * P + pc], VN = S[(HF_V + 1) * P + pc], VU = S[(HF_V + 2) * P + pc];
-      double gLoR, dLoR, gLaR, dLaR, gLoT, dLoT, gLaT, dLaT;
-      double gLoE, dLoE, gLaE, dLaE, gLoN, dLoN, gLaN, dLaN, gLoU, dLoU, gLaU, dLaU;
-      lon_of(HF_R, gLoR, dLoR);
-      lat_of(HF_R, gLaR, dLaR);
-      lon_of(HF_T, gLoT, dLoT);
-      lat_of(HF_T, gLaT, dLaT);
-      lon_of(HF_V + 0, gLoE, dLoE);
-      lat_of(HF_V + 0, gLaE, dLaE);
-      lon_of(HF_V + 1, gLoN, dLoN);
-      lat_of(HF_V + 1, gLaN, dLaN);
-      lon_of(HF_V + 2, gLoU, dLoU);
-      lat_of(HF_V + 2, gLaU, dLaU);
-      // DivVel_C (:614-617)
-      const double DivVel = gLaN + gLoE - TanLat * VN * InvR;
-      // :688-694
-      kv(HF_R) = (R - dt * (R * DivVel + gLaR * VN + gLoR * VE) + dt * (dLoR + dLaR)) - R;
-      // :749-759, :765-777, :785-790 and the Coriolis terms of :803-813
-      double nE = VE - dt * (VN * gLaE + VE * gLoE + VE * (VU - TanLat * VN) * InvR + gLoT + gLoR * T / R) +
-                  dt * (dLoE + dLaE);
-      double nN = VN - dt * (VN * gLaN + VE * gLoN + (VN * VU + TanLat * (VE * VE)) * InvR + gLaT + gLaR * T / R) +
-                  dt * (dLoN + dLaN);
-      const double nU = VU - dt * (VN * gLaU + VE * gLoU) + dt * (dLoU + dLaU);
-      if (prm.use_coriolis) {
-        nE = nE + dt * (+CoriolisSin * VN - CoriolisCos * VU);
-        nN = nN - dt * (CentrifugalParameter * GC[4 * L.C + tid] + CoriolisSin * VE);
-      }
-      kv(HF_V + 0) = nE - VE;
-      kv(HF_V + 1) = nN - VN;
-      kv(HF_V + 2) = nU - VU;
-      // :817-823
-      kv(HF_T) = (T - dt * ((GC[2 * L.C + tid] - 1) * T * DivVel + gLaT * VN + gLoT * VE) + dt * (dLoT + dLaT)) - T;
-      // species continuity (:696-703) and vertical winds (:794-801)
+    double kv[HZ_PER], DivVel = 0.0;
+#pragma unroll
+    for (int j = 0; j < HZ_PER; ++j) kv[j] = 0.0;
 #pragma unroll 1
-      for (int s = 0; s < NS; ++s) {
-        double gLo, dLo, gLa, dLa;
-        lon_of(HF_N + s, gLo, dLo);
-        lat_of(HF_N + s, gLa, dLa);
-        const double x = S[(HF_N + s) * P + pc];
-        kv(HF_N + s) = (x - dt * (x * DivVel + gLa * VN + gLo * VE) + dt * (dLo + dLa)) - x;
-        lon_of(HF_W + s, gLo, dLo);
-        lat_of(HF_W + s, gLa, dLa);
-        const double w = S[(HF_W + s) * P + pc];
-        kv(HF_W + s) = (w - dt * (VN * gLa + VE * gLo) + dt * (dLa + dLo)) - w;
+    for (int fb = 0; fb < HZ_NSW; fb += A.batch) {
+      // slopes, a line of a field per thread
+      const int n = (min(fb + A.batch, HZ_NSW) - fb) * lines;
+      for (int w = tid; w < n; w += nthr) {
+        const int f = __umulhi(unsigned(w), A.magic), r = w - f * lines;
+        const bool lat = r >= nt;
+        const int x = lat ? r - nt : r;  // row x + 1, or column x + 1
+        const int at = lat ? x + 2 : (x + 2) * NI;
+        hz_slopes(S + (fb + f) * P + at, GP + (lat ? 2 * P : 0) + at, D + f * per + (lat ? L.NL + x : x * L.NLp),
+                  lat ? NI : 1, lat ? nl : 1, lat ? nt : nl, beta);
       }
-      // advected ions (:719-736)
-#pragma unroll 1
-      for (int s = 0; s < NADV; ++s) {
-        double gLo, dLo, gLa, dLa;
-        lon_of(HF_I + s, gLo, dLo);
-        lat_of(HF_I + s, gLa, dLa);
-        const double x = S[(HF_I + s) * P + pc];
-        kv(HF_I + s) =
-            (x - dt * (+gLa * GC[6 * L.C + tid] + gLo * GC[5 * L.C + tid]) + dt * (dLo + dLa)) - x;
+      __syncthreads();
+      // cells
+      if (cell) {
+        const double VE = S[(HF_V + 0) * P + pc], VN = S[(HF_V + 1) * P + pc];
+        if (fb == 0 && f0 >= HF_N && f0 < HF_W) {
+          // DivVel_C (:614-617), for the densities among this thread's fields
+          const double* v = S + HF_V * P + pc;
+          const double* d = D + HF_V * per;
+          DivVel = la.grad(v[P - NI], v[P], v[P + NI], d[per + dt0 - nl], d[per + dt0], d[per + dt0 + nl]) +
+                   lo.grad(v[-1], v[0], v[1], d[dl - 1], d[dl], d[dl + 1]) - row[2] * VN * InvR;
+        }
+        if (f0 < fb || f0 >= fb + A.batch) {
+          // another batch's fields
+        } else if (grp == 0) {
+          const double R = S[HF_R * P + pc], T = S[HF_T * P + pc], VU = S[(HF_V + 2) * P + pc];
+          const double TanLat = row[2];
+          // each sweep's advection and diffusion as it is formed; pE, pN: the pressure gradients
+          double gLo, gLa, dd;
+          sweeps(HF_R, fb, gLo, gLa, dd);
+          kv[0] = dd - (gLa * VN + gLo * VE);
+          const double ToR = T / R;
+          double pE = gLo * ToR, pN = gLa * ToR;
+          sweeps(HF_T, fb, gLo, gLa, dd);
+          kv[1] = dd - (gLa * VN + gLo * VE);
+          pE = gLo + pE;
+          pN = gLa + pN;
+          sweeps(HF_V + 0, fb, gLo, gLa, dd);
+          DivVel = gLo;
+          kv[2] = dt * (dd - (VN * gLa + VE * gLo + VE * (VU - TanLat * VN) * InvR + pE));
+          sweeps(HF_V + 1, fb, gLo, gLa, dd);
+          // DivVel_C (:614-617)
+          DivVel = gLa + DivVel - TanLat * VN * InvR;
+          // :749-759, :765-777, :785-790 and the Coriolis terms of :803-813
+          kv[3] = dt * (dd - (VN * gLa + VE * gLo + (VN * VU + TanLat * (VE * VE)) * InvR + pN));
+          // :688-694, :817-823
+          kv[0] = dt * (kv[0] - R * DivVel);
+          kv[1] = dt * (kv[1] - (value(0) - 1) * T * DivVel);
+          sweeps(HF_V + 2, fb, gLo, gLa, dd);
+          kv[4] = dt * (dd - (VN * gLa + VE * gLo));
+          if (prm.use_coriolis) {
+            const double SinLat = row[0], CosLat = row[1];
+            const double CoriolisSin = SinLat * 2 * prm.omega_body;
+            const double CoriolisCos = CosLat * 2 * prm.omega_body;
+            const double CentrifugalParameter = (prm.omega_body * prm.omega_body) * CosLat * SinLat;
+            kv[2] = kv[2] + dt * (CoriolisSin * VN - CoriolisCos * VU);
+            kv[3] = kv[3] - dt * (CentrifugalParameter * value(1) + CoriolisSin * VE);
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < HZ_PER; ++j) {
+            if (j >= nf) continue;
+            const int f = f0 + j;
+            double gLo, gLa, dd;
+            sweeps(f, fb, gLo, gLa, dd);
+            // species continuity (:696-703), vertical winds (:794-801), advected ions (:719-736)
+            double an = VN, ae = VE;
+            if (f >= HF_I) {
+              ae = value(2);
+              an = value(3);
+            }
+            double adv = gLa * an + gLo * ae;
+            if (f < HF_W) adv = fma(S[f * P + pc], DivVel, adv);
+            kv[j] = dt * (dd - adv);
+          }
+        }
       }
+      __syncthreads();  // every read of this batch's slopes, and at last of this stage's state, is done
     }
-    __syncthreads();  // every read of this stage's state is done
+    // update
+    const double ca = (st == 1 || st == 2) ? 2.0 : 1.0, cx = (st < 2) ? 0.5 : 1.0;
     if (cell) {
 #pragma unroll
-      for (int f = 0; f < HZ_NSW; ++f) {
-        const double o = src_of(f)[pc];
-        const double kf = Kc[f * L.C + tid];
-        double nx;
-        if (st == 0) {
-          acc[f] = kf;
-          nx = 0.5 * kf + o;
-        } else if (st == 1) {
-          acc[f] = acc[f] + 2.0 * kf;
-          nx = 0.5 * kf + o;
-        } else if (st == 2) {
-          acc[f] = acc[f] + 2.0 * kf;
-          nx = kf + o;
-        } else {
-          acc[f] = acc[f] + kf;
-          nx = o + (1.0 / 6.0) * acc[f];
-        }
-        S[f * P + pc] = nx;
+      for (int j = 0; j < HZ_PER; ++j) {
+        if (j >= nf) continue;
+        const double a = (st == 0) ? kv[j] : acc(j) + ca * kv[j];
+        if (st < 3) acc(j) = a;
+        const double o = orig(j);
+        S[(f0 + j) * P + pc] = (st == 3) ? o + (1.0 / 6.0) * a : cx * kv[j] + o;
       }
     }
     __syncthreads();
   }
 
   // ---------------------------------------------------------------- store
-  auto out = [&](double* a, int f, int nf) { return a + ((int64_t(b) * nf + f) * NK + (k + 1)) * P + pc; };
+  auto out = [&](double* a, int f, int n) { return a + ((int64_t(b) * n + f) * NK + (k + 1)) * PG + pg; };
   if (cell) {
-    *out(B.rho, 0, 1) = S[HF_R * P + pc];
-    for (int d = 0; d < 3; ++d) *out(B.velocity, d, 3) = S[(HF_V + d) * P + pc];
-    const double Tn = S[HF_T * P + pc];
-    if (B.temp_source)
-      B.temp_source[((int64_t(b) * na + (k - 1)) * nt + (cj - 1)) * nl + (ci - 1)] = Tn - src_of(HF_T)[pc];
-    *out(B.temperature, 0, 1) = Tn;
     bool neg = false;
-    for (int s = 0; s < NS; ++s) {
-      *out(B.vert_vel, s, NS) = S[(HF_W + s) * P + pc];
-      const double nd = S[(HF_N + s) * P + pc];
-      neg = neg || nd < 0.0;
-      *out(B.ndensity_s, s, GITM_NSPECIES_TOTAL) = nd;
+#pragma unroll
+    for (int j = 0; j < HZ_PER; ++j) {
+      if (j >= nf) continue;
+      const int f = f0 + j;
+      const double v = S[f * P + pc];
+      if (f >= HF_I) continue;  // the ions below
+      double* o = f == HF_R ? out(B.rho, 0, 1) : f == HF_T ? out(B.temperature, 0, 1)
+                : f < HF_N ? out(B.velocity, f - HF_V, 3)
+                : f < HF_W ? out(B.ndensity_s, f - HF_N, GITM_NSPECIES_TOTAL) : out(B.vert_vel, f - HF_W, NS);
+      if (f == HF_T && B.temp_source)
+        B.temp_source[((int64_t(b) * na + (k - 1)) * nt + (cj - 1)) * nl + (ci - 1)] = v - orig(j);
+      if (f >= HF_N && f < HF_W) neg = neg || v < 0.0;
+      *o = v;
     }
     if (neg) atomicOr(&A.status[b], GITM_ST_NEG_DENSITY);  // the reference stops (:359-372)
-    if (prm.use_ion_advection) {
+    if (prm.use_ion_advection && grp == HZ_GRP - 1) {
+      const double CosLat = row[1], TanLat = row[2];
       const bool div = prm.use_improved_ion_advection != 0;
       double change = 0.0;
       if (div) {
@@ -325,9 +402,8 @@ __global__ void __launch_bounds__(NT, MINB) hz_step_kernel(const HzArgs A) {
         // iDir of IVelocityPar(iDir) plus the latitude and radial terms
         const double* VI = prm.non_magnetic ? B.ivelocity : B.ivelocity_par;
         auto vi = [&](int d, int i, int j, int kk) {
-          return VI[((int64_t(b) * 3 + d) * NK + (kk + 1)) * P + int64_t(j + 1) * NI + (i + 1)];
+          return VI[((int64_t(b) * 3 + d) * NK + (kk + 1)) * PG + int64_t(j + 1) * NG + (i + 1)];
         };
-        const double InvR = GC[3 * L.C + tid];
         double D = 0.0;
         double g = 0.0;
         if (nl > 1) {
@@ -350,9 +426,9 @@ __global__ void __launch_bounds__(NT, MINB) hz_step_kernel(const HzArgs A) {
         D = D - tl * vi(1, ci, cj, k) * InvR;
         g = 0.0;
         if (na > 1) {
-          const double* Rg = B.radial_distance + int64_t(b) * V + int64_t(cj + 1) * NI + (ci + 1);
-          const double Drp = Rg[(k + 2) * P] - Rg[(k + 1) * P];
-          const double Drm = Rg[(k + 1) * P] - Rg[k * P];
+          const double* Rg = B.radial_distance + int64_t(b) * V + pg;
+          const double Drp = Rg[int64_t(k + 2) * PG] - Rg[int64_t(k + 1) * PG];
+          const double Drm = Rg[int64_t(k + 1) * PG] - Rg[int64_t(k) * PG];
           const double DrmOverDrp = Drm / Drp;
           const double Drr2 = DrmOverDrp * DrmOverDrp;
           const double Bottom = Drm * (1 + DrmOverDrp);
@@ -388,15 +464,15 @@ __global__ void __launch_bounds__(NT, MINB) hz_step_kernel(const HzArgs A) {
       B.idensity_s[off + int64_t(GITM_NIONS - 1) * V] = e;
     };
     const int64_t base = int64_t(b) * GITM_NIONS * V;
-    for (int c = tid; c < P; c += NT) {
-      const int i = c % NI - 1, j = c / NI - 1;
+    for (int c = tid; c < PG; c += nthr) {
+      const int i = c % NG - 1, j = c / NG - 1;
       if (i >= 1 && i <= nl && j >= 1 && j <= nt) continue;
-      esum(base + (k + 1) * P + c);
+      esum(base + int64_t(k + 1) * PG + c);
     }
     if (k == 1)
-      for (int64_t c = tid; c < 2 * P; c += NT) esum(base + c);  // altitudes -1, 0
+      for (int64_t c = tid; c < 2 * PG; c += nthr) esum(base + c);  // altitudes -1, 0
     if (k == na)
-      for (int64_t c = tid; c < 2 * P; c += NT) esum(base + (na + 2) * P + c);  // nAlts+1, nAlts+2
+      for (int64_t c = tid; c < 2 * PG; c += nthr) esum(base + int64_t(na + 2) * PG + c);  // nAlts+1, nAlts+2
   }
 }
 
@@ -515,11 +591,31 @@ cudaError_t hz_exchange_launch(const GitmHzExchange& x, uint32_t* status, cudaSt
   return cudaGetLastError();
 }
 
-size_t hz_smem_bytes(int n_lons, int n_lats) { return size_t(hz_layout(n_lons, n_lats).stride) * sizeof(double); }
+constexpr size_t HZ_MAX_SMEM = 227 * 1024;  // of a CTA on sm_100
+
+static size_t hz_smem(int n_lons, int n_lats, int batch, bool keep) {
+  return size_t(hz_layout(n_lons, n_lats, batch, keep).stride) * sizeof(double);
+}
+
+// Orig and the accumulators in shared memory, with at least a group's fields
+// of slopes, where that fits.
+static bool hz_keep(int n_lons, int n_lats) { return hz_smem(n_lons, n_lats, HZ_PER, true) <= HZ_MAX_SMEM; }
+
+// All fields' slopes at once where they fit, else as many as do.
+static int hz_batch(int n_lons, int n_lats) {
+  const bool keep = hz_keep(n_lons, n_lats);
+  int batch = HZ_PER * HZ_GRP;
+  while (batch > HZ_PER && hz_smem(n_lons, n_lats, batch, keep) > HZ_MAX_SMEM) batch -= HZ_PER;
+  return batch;
+}
+
+size_t hz_smem_bytes(int n_lons, int n_lats) {
+  return hz_smem(n_lons, n_lats, hz_batch(n_lons, n_lats), hz_keep(n_lons, n_lats));
+}
 
 int hz_threads(int n_lons, int n_lats) {
   const int c = n_lons * n_lats;
-  return c <= 96 ? 96 : (c <= 128 ? 128 : (c <= 256 ? 256 : 0));
+  return c <= 256 ? HZ_GRP * ((c + 31) / 32 * 32) : 0;
 }
 
 cudaError_t hz_launch(const GitmHzParams& prm, const GitmHzBlocks& b, double dt, uint32_t* status,
@@ -530,10 +626,15 @@ cudaError_t hz_launch(const GitmHzParams& prm, const GitmHzBlocks& b, double dt,
   a.dt = dt;
   a.status = status;
   const int nt = hz_threads(b.n_lons, b.n_lats);
+  a.group = nt / HZ_GRP;
+  a.batch = hz_batch(b.n_lons, b.n_lats);
+  a.magic = unsigned(((uint64_t(1) << 32) + (b.n_lons + b.n_lats) - 1) / (b.n_lons + b.n_lats));
   const size_t smem = hz_smem_bytes(b.n_lons, b.n_lats);
-  // 96 threads: 9 x 9 blocks (GITM's usual size) at 4 CTAs per SM
-  const void* fn = (nt == 96) ? (const void*)hz_step_kernel<96, 4>
-                 : (nt == 128) ? (const void*)hz_step_kernel<128, 3> : (const void*)hz_step_kernel<256, 1>;
+  // up to 96 cells (9 x 9 blocks, GITM's usual size): two CTAs or more per SM
+  const bool keep = hz_keep(b.n_lons, b.n_lats);
+  const void* fn = keep ? (nt <= 384   ? (const void*)hz_step_kernel<384, 2, true>
+                           : nt <= 768 ? (const void*)hz_step_kernel<768, 1, true> : (const void*)hz_step_kernel<1024, 1, true>)
+                        : (const void*)hz_step_kernel<1024, 1, false>;
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
   if (e != cudaSuccess) return e;
   void* args[] = {&a};
