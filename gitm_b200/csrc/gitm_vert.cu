@@ -1469,33 +1469,58 @@ extern "C" int gitm_vert_advance_1d(GitmVertCtx* ctx, const GitmModVerticalBatch
 
 // ------------------------------------------------------------------ CFL
 // calc_timestep_vertical, calc_timestep.f90:109-145: cMax on cells
-// 0..nAlts+1 and the per-column CFL step, reduced to one minimum.  Positive
-// doubles order like their bit patterns, so the minimum is an integer atomicMin.
-__global__ void cfl_kernel(GitmColumnBatch b, const double* dalt, int gpc, double cfl, int ion,
-                           unsigned long long* out) {
-  const int64_t c = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+// 0..nAlts+1 and the CFL step of every column, reduced to one minimum.
+// Positive doubles order like their bit patterns, so the minimum is an
+// integer atomicMin.
+//
+// Bound by HBM: ten doubles per cell.  A warp takes 32 columns of every
+// CFL_ROWS-th altitude, so a block has about seven independent rows of loads
+// per thread where one thread per column walked 52 of them in turn with too
+// few in flight.  The division rounds monotonically, so the smallest of the
+// rows' steps is the column's step.  A block is 32 columns, the group whose
+// minimum is dropped if it is not positive.  1 degree globe (64,800 columns x
+// 50), the call with its transfer: 131 -> 96 us.  Four blocks per SM at 64
+// registers; at 92, 48 and 40 registers (2, 5, 6 blocks) it took 112, 102 and
+// 110 us, and loads a row ahead of their use, 4 or 16 rows gained nothing.
+constexpr int CFL_ROWS = 8;
+
+__global__ void __launch_bounds__(32 * CFL_ROWS, 4) cfl_kernel(GitmColumnBatch b, const double* dalt, int gpc, double cfl,
+                                                            int ion, unsigned long long* out) {
+  __shared__ double part[CFL_ROWS][32];
+  const int64_t c = int64_t(blockIdx.x) * 32 + threadIdx.x;
   double dtl = 1.0e32;
   if (c < b.n_cols) {
     const int nA = b.n_alts, G = nA + 4;
     const int64_t n = b.n_cols;
     double mxr = 0.0, mxi = 0.0;
-    for (int g = 1; g <= nA + 2; ++g) {
-      double mx = fabs(b.vert_vel[(int64_t(0) * G + g) * n + c]);
-      for (int s = 1; s < NS; ++s) mx = fmax(mx, fabs(b.vert_vel[(int64_t(s) * G + g) * n + c]));
+#pragma unroll 1
+    for (int g = 1 + threadIdx.y; g <= nA + 2; g += CFL_ROWS) {
+      const bool in = g >= 2 && g <= nA + 1;
+      double w[NS];
+#pragma unroll
+      for (int s = 0; s < NS; ++s) w[s] = fabs(b.vert_vel[(int64_t(s) * G + g) * n + c]);
+      const double wi = ion && in ? fabs(b.ivel_up[int64_t(g) * n + c]) : 0.0;
+      const double dz = gpc && in ? dalt[int64_t(g) * n + c] : dalt[g];
       const double snd = sqrt(b.gamma[int64_t(g) * n + c] * b.temperature[int64_t(g) * n + c]);
+      double mx = w[0];
+#pragma unroll
+      for (int s = 1; s < NS; ++s) mx = fmax(mx, w[s]);
       const double cm = mx + snd;
       if (b.cmax) b.cmax[int64_t(g) * n + c] = cm;
-      if (g >= 2 && g <= nA + 1) {
-        const double dz = gpc ? dalt[int64_t(g) * n + c] : dalt[g];
+      if (in) {
         mxr = fmax(mxr, cm / dz);
-        if (ion) mxi = fmax(mxi, (fabs(b.ivel_up[int64_t(g) * n + c]) + snd) / dz);
+        if (ion) mxi = fmax(mxi, (wi + snd) / dz);
       }
     }
     dtl = fmin(dtl, cfl / mxr);
     if (ion) dtl = fmin(dtl, cfl / mxi);
   }
+  part[threadIdx.y][threadIdx.x] = dtl;
+  __syncthreads();
+  if (threadIdx.y) return;
+  for (int r = 1; r < CFL_ROWS; ++r) dtl = fmin(dtl, part[r][threadIdx.x]);
   for (int off = 16; off > 0; off >>= 1) dtl = fmin(dtl, __shfl_xor_sync(0xffffffffu, dtl, off));
-  if ((threadIdx.x & 31) == 0 && dtl > 0.0) atomicMin(out, __double_as_longlong(dtl));
+  if (threadIdx.x == 0 && dtl > 0.0) atomicMin(out, __double_as_longlong(dtl));
 }
 
 extern "C" int gitm_vert_cfl_dt(GitmVertCtx* ctx, const GitmColumnBatch* members, int n_members, double cfl,
@@ -1503,21 +1528,22 @@ extern "C" int gitm_vert_cfl_dt(GitmVertCtx* ctx, const GitmColumnBatch* members
   if (!ctx || !dt_out || (n_members > 0 && !members)) return set_err(ctx, GITM_ERR_ARG, "bad arguments");
   CUDA_TRY(ctx, cudaSetDevice(ctx->device));
   if (!ctx->d_scalar) CUDA_TRY(ctx, cudaMalloc(&ctx->d_scalar, sizeof(double)));
-  const double init = 1.0e32;
-  CUDA_TRY(ctx, cudaMemcpy(ctx->d_scalar, &init, sizeof init, cudaMemcpyHostToDevice));
+  // all ones: above every positive double, so an untouched word means no step
+  CUDA_TRY(ctx, cudaMemsetAsync(ctx->d_scalar, 0xff, sizeof(double)));
   for (int m = 0; m < n_members; ++m) {
     const GitmColumnBatch& b = members[m];
     if (b.n_cols <= 0) continue;
     if (!b.vert_vel || !b.gamma || !b.temperature || !b.dalt_c || (ctx->params.use_ion_advection && !b.ivel_up))
       return set_err(ctx, GITM_ERR_ARG, "cfl needs vert_vel, gamma, temperature, dalt_c (and ivel_up)");
-    const int threads = 256;
-    const unsigned blocks = unsigned((b.n_cols + threads - 1) / threads);
-    cfl_kernel<<<blocks, threads>>>(b, b.dalt_c, b.grid_per_column, cfl, ctx->params.use_ion_advection,
+    const unsigned blocks = unsigned((b.n_cols + 31) / 32);
+    cfl_kernel<<<blocks, dim3(32, CFL_ROWS)>>>(b, b.dalt_c, b.grid_per_column, cfl, ctx->params.use_ion_advection,
                                     reinterpret_cast<unsigned long long*>(ctx->d_scalar));
     CUDA_TRY(ctx, cudaGetLastError());
   }
-  double local = 0.0;
-  CUDA_TRY(ctx, cudaMemcpy(&local, ctx->d_scalar, sizeof local, cudaMemcpyDeviceToHost));
+  unsigned long long word = 0;
+  CUDA_TRY(ctx, cudaMemcpy(&word, ctx->d_scalar, sizeof word, cudaMemcpyDeviceToHost));
+  double local = 1.0e32;
+  if (word != ~0ull) std::memcpy(&local, &word, sizeof local);
   // DtLocal = min(DtLocal, DtEnd); Dt = min(Dt, DtVertical)  (calc_timestep.f90:141-147)
   *dt_out = std::min(dt_in, std::min(local, dt_end));
   return GITM_OK;
