@@ -168,7 +168,6 @@ struct GitmVertPlan {
   Tile* d_adj_tiles = nullptr;
   size_t adj_smem = 0;
   int adj_grid = 0, adj_per_max = 0;
-  double* d_adj_scratch = nullptr;
   GitmColumnAdjoint* d_bars = nullptr;
   // the saving step kernel (its own tiles and persistent grid)
   // tile ranges whose stage states a call without saved ones forms and
@@ -613,7 +612,7 @@ static int plan_common(GitmVertPlan* P, const double* const* alt, const double* 
 static void plan_free(GitmVertPlan* P) {
   if (!P) return;
   P->pool->drain();  // what the plan launched, on any stream, is done with its memory
-  for (void* p : {(void*)P->d_adj_tiles, (void*)P->d_save_tiles, (void*)P->d_adj_scratch, (void*)P->d_adj_states,
+  for (void* p : {(void*)P->d_adj_tiles, (void*)P->d_save_tiles, (void*)P->d_adj_states,
                   (void*)P->d_bars, (void*)P->d_scratch, (void*)P->d_members, (void*)P->d_grid, (void*)P->d_status,
                   (void*)P->d_tiles})
     P->pool->put(p);
@@ -951,7 +950,7 @@ static int adjoint_chunks(GitmVertPlan* P, int64_t columns) {
   return GITM_OK;
 }
 
-// Tiles, persistent grid and scratch of the adjoint kernel for the plan.
+// Tiles and persistent grid of the adjoint kernel for the plan.
 static int adjoint_prepare(GitmVertPlan* P) {
   GitmVertCtx* ctx = P->ctx;
   if (P->adj_ready) return GITM_OK;
@@ -1000,17 +999,20 @@ static int adjoint_prepare(GitmVertPlan* P) {
   }
   const void* fn = (plan_nalts(P) == 50) ? adjoint_kernel_fn_n50() : adjoint_kernel_fn();
   CUDA_TRY(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(ctx->max_smem)));
-  int per_sm = 0;
-  CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, T, P->adj_smem));
-  per_sm = std::max(per_sm, 1);
+  // CTAs per SM: by registers, shared memory and tensor memory (the occupancy
+  // query counts a kernel that takes any tensor memory as taking all of it)
+  cudaFuncAttributes fa;
+  int regs = 0, smem = 0, reserved = 0;
+  CUDA_TRY(ctx, cudaFuncGetAttributes(&fa, fn));
+  CUDA_TRY(ctx, cudaDeviceGetAttribute(&regs, cudaDevAttrMaxRegistersPerMultiprocessor, ctx->device));
+  CUDA_TRY(ctx, cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerMultiprocessor, ctx->device));
+  CUDA_TRY(ctx, cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, ctx->device));
+  const int regs_cta = (fa.numRegs + 7) / 8 * 8 * T;
+  const int per_sm = std::max(1, std::min({512 / ADJ_TM_COLS, regs / regs_cta, int(smem / (P->adj_smem + reserved))}));
   P->adj_grid = int(std::min<size_t>(P->adj_tiles.size(), size_t(per_sm) * ctx->num_sms));
   CUDA_TRY(ctx, plan_alloc(P, &P->d_adj_tiles, P->adj_tiles.size()));
   CUDA_TRY(ctx, cudaMemcpy(P->d_adj_tiles, P->adj_tiles.data(), P->adj_tiles.size() * sizeof(Tile),
                            cudaMemcpyHostToDevice));
-  if (plan_alloc(P, &P->d_adj_scratch, size_t(P->adj_grid) * 2 * NF * T) != cudaSuccess) {
-    cudaGetLastError();
-    return set_err(ctx, GITM_ERR_NOMEM, "adjoint: cannot allocate the stage-adjoint scratch");
-  }
   CUDA_TRY(ctx, plan_alloc(P, &P->d_bars, std::max(1, P->n_members)));
   if (!kernel_for(0, GITM_SOLVER_RUSANOV, TILE_THREADS, plan_nalts(P), true))
     return set_err(ctx, GITM_ERR_ARG, "the saving step kernel is not built");
@@ -1114,7 +1116,6 @@ extern "C" int gitm_vert_plan_adjoint(GitmVertPlan* P, const GitmColumnAdjoint* 
   kp.per_max = P->adj_per_max;
   kp.dt = dt;
   kp.status = P->d_status;
-  kp.scratch = P->d_adj_scratch;
   kp.prm = ctx->params;
   const void* fn = (plan_nalts(P) == 50) ? adjoint_kernel_fn_n50() : adjoint_kernel_fn();
   auto launch = [&](int t0, int t1, const double* states, int64_t c0, int64_t n) -> int {
