@@ -162,15 +162,22 @@ __device__ __forceinline__ void species_face_flux(double rl, double rr, double p
   mflux = (up ? rl * wl : rr * wr) * nv;
 }
 
+constexpr uint32_t AUSM_TM_ND = 136;
+
 // advance_vertical_1stage_ausm (vertical_solver_ausm.f90:436-999) at interior
 // cell i with stage step dtk; emit(f, New - state) takes each new value.
 // The face fluxes of calc_all_fluxes_hydro are formed at the cell's two
 // faces in two passes over the species: the first sums the bulk face states
 // (densities, pressures, mass-weighted vertical wind), which set the Liou
 // sound speed; the second forms the species fluxes and applies them.
-template <class Emit>
+// TM: the first pass's face states are kept in the thread's tensor memory
+// (NS x 16 columns at tm) for the second, which leaves its results there; the
+// cell's densities and deviations at tm + AUSM_TM_ND, 4 columns a species.
+// Whole warps call.
+template <bool TM, class Emit>
 __device__ __forceinline__ void ausm_cell(ColCtx c, int i, const GitmVertParams& prm, double dtk,
-                                          double eddy, double ivup, Emit&& emit, uint32_t* st = nullptr) {
+                                          double eddy, double ivup, uint32_t tm, Emit&& emit,
+                                          uint32_t* st = nullptr) {
   const int nA = c.L.nAlts;
   (void)nA;
   const double logk = c_k.log_kb;
@@ -189,13 +196,6 @@ __device__ __forceinline__ void ausm_cell(ColCtx c, int i, const GitmVertParams&
   ausm_sweep(c, AS_VN4, F_VN, i, fc0, fc1, gN, dN);
   (void)gE;
   (void)gN;
-#pragma unroll
-  for (int s = 0; s < NADV; ++s) {
-    double gI, dI;
-    ausm_sweep(c, AS_I4 + s, F_I + s, i, fc0, fc1, gI, dI);
-    const double I = c.x(F_I + s, i);
-    emit(F_I + s, (I - dtk * (ivup * gI) + dtk * dI) - I);  // :857-860
-  }
 
   // cell values (:560-575, 752-790)
   double ns[NS], Rho;
@@ -234,6 +234,14 @@ __device__ __forceinline__ void ausm_cell(ColCtx c, int i, const GitmVertParams&
     }
   }
 
+  if constexpr (TM) {
+#pragma unroll
+    for (int s = 0; s < NS; ++s) {
+      tm_put(tm + AUSM_TM_ND + 4 * s, ns[s]);
+      tm_put(tm + AUSM_TM_ND + 4 * s + 2, dev[s]);
+    }
+  }
+
   // ---- pass 1: bulk face states
   double RhoLM = 0.0, RhoRM = 0.0, RhoLP = 0.0, RhoRP = 0.0;
   double PLM = 0.0, PRM = 0.0, PLP = 0.0, PRP = 0.0;
@@ -242,10 +250,11 @@ __device__ __forceinline__ void ausm_cell(ColCtx c, int i, const GitmVertParams&
   // instruction cache could not hold.  The faces' exponentials go in batches
   // and the divisions that a face's species share are taken once; with one
   // copy of the boundary passes in the kernel (409 -> 238 KB of code) 2.5
-  // degrees, 4 steps: 10.5 -> 8.5 ms
+  // degrees, 4 steps: 10.5 -> 8.5 ms; with the face states, the loop's values,
+  // K and the accumulators in tensor memory (TM) 6.9 ms
   // the density and pressure face states of each species, kept from this
-  // pass for the flux pass (per-thread memory, cached)
-  double fst[NS][8];
+  // pass for the flux pass (without TM in per-thread memory)
+  double fst[TM ? 1 : NS][8];
 #pragma unroll 1
   for (int s = 0; s < NS; ++s) {
     const double lm = c_k.log_mass[s];
@@ -257,8 +266,13 @@ __device__ __forceinline__ void ausm_cell(ColCtx c, int i, const GitmVertParams&
                          logk + tp.lm, logk + tp.rm, logk + tp.lp, logk + tp.rp};
     double e[8];
     exp_n(a, e);
+    if constexpr (TM) {
+      __syncwarp();
+      tm_put(tm + 16 * s, e);
+    } else {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) fst[s][j] = e[j];
+      for (int j = 0; j < 8; ++j) fst[s][j] = e[j];
+    }
     RhoLM = RhoLM + e[0];
     RhoRM = RhoRM + e[1];
     RhoLP = RhoLP + e[2];
@@ -272,6 +286,7 @@ __device__ __forceinline__ void ausm_cell(ColCtx c, int i, const GitmVertParams&
     WLP = WLP + e[2] * w.lp;
     WRP = WRP + e[3] * w.rp;
   }
+  if constexpr (TM) tm_put_wait();
   // bulk face winds (:1503-1530): the up component is the mass-weighted species wind
   const double ULM = WLM / RhoLM, URM = WRM / RhoRM, ULP = WLP / RhoLP, URP = WRP / RhoRP;
   const Faces fE = kt_faces(c, AS_VE, i, c.x(F_VE, i - 1), VE, c.x(F_VE, i + 1));
@@ -313,9 +328,17 @@ __device__ __forceinline__ void ausm_cell(ColCtx c, int i, const GitmVertParams&
       exp_faces(kt_faces(c, AS_LHPS + s, i, hydro_q(c, s, i - 1), hydro_q(c, s, i), hydro_q(c, s, i + 1)),
                 c.x(F_LNS + s, 0) + lnk0, h);
     const Faces w = kt_faces(c, AS_W + s, i, c.x(F_W + s, i - 1), c.x(F_W + s, i), c.x(F_W + s, i + 1));
-    double f[8];
+    double f[8], nd[4];
+    if constexpr (TM) {
+      __syncwarp();
+      tm_get(tm + 16 * s, f);
+      tm_get(tm + AUSM_TM_ND + 4 * s, nd);
+    } else {
+      nd[0] = ns[s];
+      nd[1] = dev[s];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) f[j] = fst[s][j];
+      for (int j = 0; j < 8; ++j) f[j] = fst[s][j];
+    }
     double nvM, rfM, mfM, npM, nvP, rfP, mfP, npP;
     species_face_flux(f[0], f[1], f[4], f[5], h[0], h[1], w.lm, w.rm, CSM, iCSM, kp, ku, dzdt, sh, nvM, rfM, mfM, npM);
     species_face_flux(f[2], f[3], f[6], f[7], h[2], h[3], w.lp, w.rp, CSP, iCSP, kp, ku, dzdt, sh, nvP, rfP, mfP, npP);
@@ -323,17 +346,38 @@ __device__ __forceinline__ void ausm_cell(ColCtx c, int i, const GitmVertParams&
     BulkVM = BulkVM + (f[0] + f[1]) * nvM;
     const double RhoSFlux = (AP * rfP - AM * rfM) * iVol;
     const double MomSFlux = (AP * mfP - AM * mfM) * iVol + (npP - npM) * idAltC;
-    const double RhoS = c_k.mass[s] * ns[s];
+    const double RhoS = c_k.mass[s] * nd[0];
     const double Ws = c.x(F_W + s, i);
     const double NewRhoS = RhoS - dtk * RhoSFlux;
     const double MomS = RhoS * Ws;
-    const double NewMomS = MomS - dtk * MomSFlux + dtk * (sh ? dev[s] : RhoS) * EG;
+    const double NewMomS = MomS - dtk * MomSFlux + dtk * (sh ? nd[1] : RhoS) * EG;
     double w1 = NewMomS / NewRhoS;
     w1 = w1 + hz;
     if (prm.use_coriolis) w1 = w1 + dtk * (c.sc(SC_CORI) * VE);
     w1 = w1 - dtk * (prm.thermal_diff_coef[s] * c_k.k_over_m[s]) * gT;
-    nrs[s] = NewRhoS;
-    wv[s] = w1;
+    if constexpr (TM) {
+      const double r[4] = {NewRhoS, w1, 0.0, 0.0};
+      __syncwarp();
+      tm_put(tm + 16 * s, r);
+    } else {
+      nrs[s] = NewRhoS;
+      wv[s] = w1;
+    }
+  }
+  if constexpr (TM) {
+    static_assert(NS == 6, "two groups of three species");
+    tm_put_wait();
+#pragma unroll
+    for (int s = 0; s < NS; s += 3) {
+      double u[4], v[4], w[4];
+      tm_get(tm + 16 * s, tm + 16 * s + 16, tm + 16 * s + 32, u, v, w);
+      nrs[s] = u[0];
+      nrs[s + 1] = v[0];
+      nrs[s + 2] = w[0];
+      wv[s] = u[1];
+      wv[s + 1] = v[1];
+      wv[s + 2] = w[1];
+    }
   }
   BulkVP = BulkVP / (RhoLP + RhoRP);
   BulkVM = BulkVM / (RhoLM + RhoRM);
@@ -407,6 +451,14 @@ __device__ __forceinline__ void ausm_cell(ColCtx c, int i, const GitmVertParams&
   const double NewPress =
       (NewTotalEnergy - 0.5 * NewRho * (NewVU * NewVU + NewVN * NewVN + NewVE * NewVE)) * (gam - 1.0);
   emit(F_T, NewPress / (KB * NewNT) - T);
+
+#pragma unroll
+  for (int s = 0; s < NADV; ++s) {
+    double gI, dI;
+    ausm_sweep(c, AS_I4 + s, F_I + s, i, fc0, fc1, gI, dI);
+    const double I = c.x(F_I + s, i);
+    emit(F_I + s, (I - dtk * (ivup * gI) + dtk * dI) - I);  // :857-860
+  }
 }
 
 }  // namespace gv

@@ -770,6 +770,7 @@ __device__ __forceinline__ void rusanov_slopes_cell(ColCtx c, int i, double beta
 
 }  // namespace gv
 
+#include "vert_tmem.cuh"
 #include "vert_ausm.cuh"
 
 namespace gv {
@@ -821,6 +822,25 @@ __global__ void __launch_bounds__(NT, MINB) vert_step_kernel(const KParams kp) {
   double* accg = ACC_GLOBAL ? slot + tid : nullptr;
   double* const ogb = OG ? slot + size_t(NF) * NT : nullptr;  // Orig of column cl at ogb + cl * orig_doubles
   const double inv_vert_tau = 1.0 / prm.vert_tau;  // 1 / VertTau without damping
+  // The AUSM shape with one CTA per SM: the face states of the flux passes,
+  // the stage's K and the RK accumulators in tensor memory, three warps to a
+  // quarter of its lanes.  K and the accumulators take the face states'
+  // columns once those are read, so that Orig is fetched in one batch.
+  constexpr bool TM = SOLVER == GITM_SOLVER_AUSM && NT == 384 && MINB == 1 && OG;
+  constexpr uint32_t TMW = 168, TM_KV = 0, TM_AC = 96;  // columns of a warp; K; accumulators (20 doubles each)
+  uint32_t tm_base = 0, tm = 0;
+  if constexpr (TM) {
+    static_assert(!TM || (3 * TMW <= 512 && TM_AC >= 16 * NS && TM_AC + 40 <= AUSM_TM_ND && AUSM_TM_ND + 4 * NS + 4 <= TMW), "tensor memory of a warp");
+    if (wid == 0) {
+      const uint32_t where = uint32_t(__cvta_generic_to_shared(sm));
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(where) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    __syncthreads();
+    tm_base = *reinterpret_cast<volatile uint32_t*>(sm);
+    tm = tm_base + (uint32_t(wid & 3) << 21) + uint32_t(wid >> 2) * TMW;
+    __syncthreads();
+  }
 
   for (int tix = blockIdx.x; tix < kp.n_tiles; tix += gridDim.x) {
     const Tile tile = kp.tiles[tix];
@@ -1094,7 +1114,43 @@ __global__ void __launch_bounds__(NT, MINB) vert_step_kernel(const KParams kp) {
         // exact, so fma(ca, K, prev) rounds like prev + ca K
         const double ca = (k == 1 || k == 2) ? 2.0 : 1.0;
         const double cx = (k < 2) ? 0.5 : (k == 2) ? 1.0 : 1.0 / 6.0;
-        if (item) {
+        if constexpr (TM) {
+          if (wid * 32 < nitems) {  // the idle lanes of the last warp repeat a cell and store nothing
+            ColCtx c = ctx(my_cl);
+            const int i = my_i;
+            ausm_cell<true>(c, i, prm, (k == 2) ? dt : 0.5 * dt, eddy, ivup, tm,
+                            [&](int f, double kval) { tm_put(tm + TM_KV + 2 * f, kval); }, &sst[my_cl]);
+            double o[20];
+            const double* og = ogb + size_t(my_cl) * operc + i + 1;
+#pragma unroll
+            for (int f = 0; f < NF; ++f) o[f] = og[f * G];
+            tm_put_wait();
+            double* xn = c.col + nxo + 1;
+            // Stage(k+2) = Stage1 + (New - state), and the final combination
+            // (1/3)(-Stage1 + Stage2 + 2 Stage3 + Stage4 + (New - state))
+            // accumulated in the reference's order (vertical_solver_ausm.f90:167-189,381-420)
+#pragma unroll
+            for (int f0 = 0; f0 < NF; f0 += 4) {
+              double kv[4], ac[4];
+              tm_get(tm + TM_KV + 2 * f0, kv);
+              if (k > 0) tm_get(tm + TM_AC + 2 * f0, ac);
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                if (f0 + j >= NF) continue;
+                double x1 = o[f0 + j] + kv[j];
+                if (k == 0)
+                  ac[j] = -1.0 * o[f0 + j] + x1;
+                else if (k < 3)
+                  ac[j] = (k == 1) ? ac[j] + 2.0 * x1 : ac[j] + x1;
+                else
+                  x1 = (1.0 / 3.0) * (ac[j] + kv[j]);
+                if (item) xn[(f0 + j) * G + i] = x1;
+              }
+              if (k < 3) tm_put(tm + TM_AC + 2 * f0, ac);
+            }
+            tm_put_wait();
+          }
+        } else if (item) {
           ColCtx c = ctx(my_cl);
           const int i = my_i;
           double* xn = c.col + nxo + 1;  // next buffer, xn[f*G + i]
@@ -1128,7 +1184,7 @@ __global__ void __launch_bounds__(NT, MINB) vert_step_kernel(const KParams kp) {
           };
           if constexpr (SOLVER == GITM_SOLVER_AUSM) {
             // advance_vertical_1stage_ausm with DtIn = Dt/2, Dt/2, Dt, Dt/2
-            ausm_cell(c, i, prm, (k == 2) ? dt : 0.5 * dt, eddy, ivup, emit, &sst[my_cl]);
+            ausm_cell<false>(c, i, prm, (k == 2) ? dt : 0.5 * dt, eddy, ivup, 0u, emit, &sst[my_cl]);
           } else {
             rusanov_cell(c, i, prm, dt, eddy, ivup, inv_vert_tau, emit, &sst[my_cl]);
           }
@@ -1311,6 +1367,9 @@ __global__ void __launch_bounds__(NT, MINB) vert_step_kernel(const KParams kp) {
       if (w) kp.status[gcol] |= w;
     }
     __syncthreads();
+  }
+  if constexpr (TM) {
+    if (wid == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tm_base));
   }
 }
 
