@@ -81,16 +81,48 @@ __device__ __forceinline__ void ausm_prefix(ColCtx c, int lane) {
   }
 }
 
-// Phase A2: slope of AUSM field f at cell i (0..nAlts+1).
-__device__ __forceinline__ double ausm_slope(ColCtx c, int f, int i, double beta) {
+// Phase A2: the 32 slopes at cell i (0..nAlts+1): 2nd-order "kt" slopes, and
+// the 4th-order form of the last five (2nd-order at cells 0 and nAlts+1).  A
+// species' values are read once for its density and pressure slopes, and the
+// grid's coefficients once for all, ahead of the stores they would otherwise
+// be read again after (2.5 degrees, 4 steps: 6.94 -> 5.96 ms).
+__device__ __forceinline__ void ausm_slopes_cell(ColCtx c, int i, double beta) {
   const int nA = c.L.nAlts;
-  const double vm = ausm_field(c, f, i - 1), v0 = ausm_field(c, f, i), vp = ausm_field(c, f, i + 1);
-  const bool fourth = (f >= AS_T4) && i >= 1 && i <= nA;
-  if (!fourth) return limiter_mc((vp - v0) * c.g(GC_IDF, i + 1), (v0 - vm) * c.g(GC_IDF, i), beta);
-  const double vmm = ausm_field(c, f, i - 2), vpp = ausm_field(c, f, i + 2);
-  const double up = c.g(GC_H2, i + 1) * (0.6250000 * (vp - v0) - 0.0416667 * (vpp - vm));
-  const double dn = c.g(GC_H2, i) * (0.6250000 * (v0 - vm) - 0.0416667 * (vp - vmm));
-  return limiter_mc(up, dn, beta);
+  const double id1 = c.g(GC_IDF, i + 1), id0 = c.g(GC_IDF, i);
+  const bool end = i == 0 || i == nA + 1;
+  const double h1 = end ? 0.0 : c.g(GC_H2, i + 1), h0 = end ? 0.0 : c.g(GC_H2, i);
+  double* const sl = &c.dl(0, i);
+  const int pd = c.L.PD;
+  auto kt = [&](double vm, double v0, double vp) { return limiter_mc((vp - v0) * id1, (v0 - vm) * id0, beta); };
+  const double* lt = c.col + c.L.LT + i + 1;
+  const double* q = c.col + c.L.QS + i + 1;
+  const double ltm = lt[-1], lt0 = lt[0], ltp = lt[1];
+  const double qm = q[i > 0 ? -1 : 0], q0 = q[0], qp = q[1], qb = c.sc(SC_QB);
+#pragma unroll 2
+  for (int s = 0; s < NS; ++s) {
+    const double lm = c.x(F_LNS + s, i - 1), l0 = c.x(F_LNS + s, i), lp = c.x(F_LNS + s, i + 1);
+    const double wm = c.x(F_W + s, i - 1), w0 = c.x(F_W + s, i), wp = c.x(F_W + s, i + 1);
+    const double m = c_k.mass[s];
+    const double a = kt(lm, l0, lp), b = kt(lm + ltm, l0 + lt0, lp + ltp);
+    const double h = kt(i > 0 ? m * qm : qb, m * q0, m * qp), w = kt(wm, w0, wp);
+    sl[(AS_LRHOS + s) * pd] = a;
+    sl[(AS_LPS + s) * pd] = b;
+    sl[(AS_LHPS + s) * pd] = h;
+    sl[(AS_W + s) * pd] = w;
+  }
+  sl[AS_GAM * pd] = kt(c.gm(i - 1), c.gm(i), c.gm(i + 1));
+  const int ip2 = min(i + 2, nA + 2), im2 = max(i - 2, -1);
+#pragma unroll
+  for (int k = 0; k < 5; ++k) {
+    const int f = k == 0 ? F_T : k < 3 ? F_VE + k - 1 : F_I + k - 3;
+    const double vmm = c.x(f, im2), vm = c.x(f, i - 1), v0 = c.x(f, i), vp = c.x(f, i + 1), vpp = c.x(f, ip2);
+    const double u2 = (vp - v0) * id1, d2 = (v0 - vm) * id0;
+    const double u4 = h1 * (0.6250000 * (vp - v0) - 0.0416667 * (vpp - vm));
+    const double d4 = h0 * (0.6250000 * (v0 - vm) - 0.0416667 * (vp - vmm));
+    if (k == 1 || k == 2) sl[(AS_VE + k - 1) * pd] = limiter_mc(u2, d2, beta);
+    sl[(AS_T4 + k) * pd] = limiter_mc(end ? u2 : u4, end ? d2 : d4, beta);
+  }
+  static_assert(AS_VE4 == AS_T4 + 1 && AS_VN4 == AS_T4 + 2 && AS_I4 == AS_T4 + 3 && F_VN == F_VE + 1, "the order of the fields");
 }
 
 // kt face values of a field at the lower (M) and upper (P) faces of cell i:

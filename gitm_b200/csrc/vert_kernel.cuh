@@ -1089,9 +1089,7 @@ __global__ void __launch_bounds__(NT, MINB) vert_step_kernel(const KParams kp) {
           // threads over cells 0..nAlts+1 of every column
           for (int j = tid; j < nc * (nA + 2); j += NT) {
             const int cl = j / (nA + 2), i = j - cl * (nA + 2);
-            ColCtx c = ctx(cl);
-#pragma unroll 4
-            for (int f = 0; f < NSLOPE_AUSM; ++f) c.dl(f, i) = ausm_slope(c, f, i, prm.beta_limiter);
+            ausm_slopes_cell(ctx(cl), i, prm.beta_limiter);
           }
         } else {
           // limited slopes of the 18 swept fields on cells 0..nAlts+1,
