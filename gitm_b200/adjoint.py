@@ -108,7 +108,7 @@ class StepRunner:
         """Adjoint of one step taken from `state`: returns (xbar, eddy_bar,
         heating_scale_bar).  ybar: dict of output adjoints (None = zero);
         saved: the buffer step_saving filled for this step, or None (the
-        adjoint kernel then recomputes the stage states)."""
+        saving step then runs ahead of the adjoint kernel)."""
         self._load(state, eddy, heating_scale)
         bars = {}
         for k in STATE:

@@ -252,8 +252,8 @@ static void fill_consts(Consts& k) {
 // where the RK accumulator lives.  The small CTAs keep it in a per-CTA slot
 // of global scratch (L2-resident under their persistent grid) so that two or
 // three CTAs share an SM and overlap each other's barrier phases.  The AUSM
-// solver's 384-thread shape also keeps Orig there (orig_global: 6 columns of
-// its larger slot instead of 4).  The Rusanov solver's 512-thread shape is
+// solver's 384-thread shape keeps Orig there (orig_global: 6 columns of its
+// larger slot instead of 4) and the accumulators in tensor memory.  The Rusanov solver's 512-thread shape is
 // the tile kernel (vert_tile.cuh), which holds both in tensor memory.
 // solver -1: any solver.
 struct Shape { int threads, solver, min_blocks; bool acc_global, orig_global, tile; };

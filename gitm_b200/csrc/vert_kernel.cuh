@@ -807,7 +807,8 @@ struct KParams {
 // compile-time constants; NA = 0 reads nAlts from the member.
 // OG (with ACC_GLOBAL): Orig lives in the CTA's slot of global scratch after
 // the accumulators (coalesced, L2-resident, read-only within a step), so a
-// column needs 8 KB less shared memory and more columns share an SM.
+// column needs 8 KB less shared memory and more columns share an SM; its
+// 384-thread AUSM shape has the accumulators in tensor memory instead.
 template <int IO, int NT, int MINB, bool ACC_GLOBAL, int SOLVER, int NA = 0, bool OG = false>
 __global__ void __launch_bounds__(NT, MINB) vert_step_kernel(const KParams kp) {
   static_assert(!OG || ACC_GLOBAL, "Orig in global scratch goes with the accumulators there");

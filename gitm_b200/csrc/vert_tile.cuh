@@ -8,8 +8,8 @@
 //
 //  * One copy of the stage state in shared memory.  What only one thread
 //    ever touches -- Orig, the RK accumulator and the stage's increments of
-//    its cell, 57 doubles -- lives in tensor memory, which nothing else here
-//    uses: 256 KB per SM, 64 doubles for each of 512 threads, written and
+//    its cell, 57 doubles -- lives in tensor memory, idle otherwise without a
+//    contraction on the path: 256 KB per SM, 64 doubles for each of 512 threads, written and
 //    read by the thread's own warp (tcgen05.st / tcgen05.ld).  A column then
 //    needs 20 KB of shared memory at 50 altitudes.  A stage is three phases:
 //      P  set_vertical_bcs on every column and the limited slopes
