@@ -1759,7 +1759,9 @@ extern "C" int gitm_vert_advance_fortran(GitmVertCtx* ctx, const GitmFortranStat
       CUDA_TRY(ctx, ctx->pool->get(&p, all.size() * sizeof(FMap)));
       d_maps = static_cast<FMap*>(p);
       CUDA_TRY(ctx, cudaMemcpy(d_maps, all.data(), all.size() * sizeof(FMap), cudaMemcpyHostToDevice));
-      // cMax and the eddy coefficient have no outermost cells in the Fortran arrays
+      // the copies in do not reach LogNS and NDensity, which the step leaves alone in a column it refuses (the
+      // copies out give such a column zeros), nor the outermost cells of cMax and of the eddy coefficient
+      CUDA_TRY(ctx, cudaMemsetAsync(base + o_lns, 0, size_t(o_gm - o_lns) * sizeof(double), nullptr));
       CUDA_TRY(ctx, cudaMemsetAsync(base + o_cm, 0, size_t(o_ed + G * ncols - o_cm) * sizeof(double), nullptr));
       return GITM_OK;
     }();
