@@ -1367,6 +1367,9 @@ extern "C" int gitm_vert_advance_native_host(GitmVertCtx* ctx, const GitmColumnB
       if ((rc = h2d(const_cast<double*>(d.*(a.field)), b.*(a.field), rows_of(a.rows_per_cell, G)))) break;
     }
     if (rc) break;
+    // formed by the step alone, and not for a column it refuses: the copies out give such a column zeros
+    for (double* p : {d.log_ns, d.ndensity})
+      if (p) CUDA_TRY(ctx, cudaMemsetAsync(p, 0, size_t(p == d.log_ns ? NS : 1) * G * w, s_in));
     CUDA_TRY(ctx, cudaEventRecord(e_in, s_in));
     CUDA_TRY(ctx, cudaStreamWaitEvent(s_k, e_in, 0));
     const int spl = std::max(1, P->cfg.steps_per_launch);
@@ -1396,8 +1399,10 @@ extern "C" int gitm_vert_advance_native_host(GitmVertCtx* ctx, const GitmColumnB
                                         a.field == &GitmColumnBatch::temp_unit || a.field == &GitmColumnBatch::cmax))
         continue;
       if (!prm.compute_eddy && a.field == &GitmColumnBatch::eddy) continue;
-      cudaError_t e = cudaMemcpy2DAsync(b.*(a.field) + ch.c0, hp, d.*(a.field), w, w,
-                                        rows_of(a.rows_per_cell, G), cudaMemcpyDeviceToHost, s_out);
+      // the step forms cMax on cells 0 .. nAlts+1: the outermost rows stay the caller's
+      const int64_t skip = (a.field == &GitmColumnBatch::cmax) ? 1 : 0;
+      cudaError_t e = cudaMemcpy2DAsync(b.*(a.field) + skip * b.n_cols + ch.c0, hp, d.*(a.field) + skip * ch.n, w, w,
+                                        rows_of(a.rows_per_cell, G) - 2 * skip, cudaMemcpyDeviceToHost, s_out);
       if (e != cudaSuccess) rc = set_err(ctx, GITM_ERR_CUDA, "copy back: %s", cudaGetErrorString(e));
     }
   }

@@ -37,7 +37,7 @@ def fortran_call(ctx, f, on_device):
     return rc, f
 
 
-@pytest.mark.parametrize("on_device", [1], ids=["device"])
+@pytest.mark.parametrize("on_device", [1, 0], ids=["device", "host"])
 def test_fortran_arrays(on_device):
     ctx = V.VerticalContext(abi.default_params(compute_coefficients=0))
     good = fortran_arrays(synthetic.make_member(N, N_ALTS, seed=11), 1)
@@ -56,3 +56,31 @@ def test_fortran_arrays(on_device):
     for k in ("log_ns", "ndensity"):
         np.testing.assert_array_equal(out[k][li, lj], np.zeros_like(out[k][li, lj]), err_msg=k)
         assert (out[k][li - 1, lj] != before[k][li - 1, lj]).all()  # a column that was advanced
+
+
+def test_host_pointers():
+    """The host-pointer call, whose coefficients come from the step: the
+    refused column, and cMax's outermost cells, which the step does not form."""
+    ctx = V.VerticalContext(abi.default_params())
+
+    def member(seed):
+        m = synthetic.make_member(1500, N_ALTS, seed=seed)  # two chunks of columns
+        m.log_ns, m.ndensity = np.full_like(m.ndensity_s, 7.0), np.full_like(m.rho, 7.0)
+        m.cmax[:, [0, -1]] = 7.0
+        return m
+
+    V.advance_vertical_all_host(ctx, [member(13)], 2.0)
+    m = member(14)
+    bad = 1100
+    m.ndensity_s[2, 20, bad] = 0.0
+    before = m.copy()
+    with pytest.raises(V.GitmStop):
+        V.advance_vertical_all_host(ctx, [m], 2.0)
+    ctx.close()
+    for k in synthetic.Member.STATE:
+        np.testing.assert_array_equal(getattr(m, k)[..., bad], getattr(before, k)[..., bad], err_msg=k)
+    for k in ("log_ns", "ndensity"):
+        a = getattr(m, k)
+        assert (a[..., bad] == 0.0).all() and (a[..., bad - 1] != 7.0).all(), k
+    np.testing.assert_array_equal(m.cmax[:, [0, -1]], before.cmax[:, [0, -1]])
+    assert (m.cmax[:, 1:-1, :bad] > 0.0).all()
