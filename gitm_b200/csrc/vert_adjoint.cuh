@@ -1116,12 +1116,7 @@ __global__ void __launch_bounds__(NT, 1) vert_adjoint_kernel(const AParams kp) {
   constexpr int nw = NT / 32;
   const GitmVertParams& prm = kp.prm;
   const double dt = kp.dt;
-  if (wid == 0) {
-    const uint32_t where = uint32_t(__cvta_generic_to_shared(sm));
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(where), "n"(ADJ_TM_COLS)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
-  }
+  if (wid == 0) tm_alloc<ADJ_TM_COLS>(sm);
   __syncthreads();
   const uint32_t tm_base = *reinterpret_cast<volatile uint32_t*>(sm);
   const uint32_t tm = tm_base + (uint32_t(wid) << 21);  // warp w reaches the lanes 32 w ..
@@ -1621,8 +1616,7 @@ __global__ void __launch_bounds__(NT, 1) vert_adjoint_kernel(const AParams kp) {
     }
     __syncthreads();  // @phase 11
   }
-  if (wid == 0)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tm_base), "n"(ADJ_TM_COLS));
+  if (wid == 0) tm_free<ADJ_TM_COLS>(tm_base);
 }
 
 }  // namespace gv

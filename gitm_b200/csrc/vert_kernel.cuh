@@ -832,11 +832,7 @@ __global__ void __launch_bounds__(NT, MINB) vert_step_kernel(const KParams kp) {
   uint32_t tm_base = 0, tm = 0;
   if constexpr (TM) {
     static_assert(!TM || (3 * TMW <= 512 && TM_AC >= 16 * NS && TM_AC + 40 <= AUSM_TM_ND && AUSM_TM_ND + 4 * NS + 4 <= TMW), "tensor memory of a warp");
-    if (wid == 0) {
-      const uint32_t where = uint32_t(__cvta_generic_to_shared(sm));
-      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(where) : "memory");
-      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
-    }
+    if (wid == 0) tm_alloc<512>(sm);
     __syncthreads();
     tm_base = *reinterpret_cast<volatile uint32_t*>(sm);
     tm = tm_base + (uint32_t(wid & 3) << 21) + uint32_t(wid >> 2) * TMW;
@@ -1368,7 +1364,7 @@ __global__ void __launch_bounds__(NT, MINB) vert_step_kernel(const KParams kp) {
     __syncthreads();
   }
   if constexpr (TM) {
-    if (wid == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tm_base));
+    if (wid == 0) tm_free<512>(tm_base);
   }
 }
 

@@ -470,11 +470,7 @@ __global__ void __launch_bounds__(TILE_THREADS, 1) vert_tile_kernel(const KParam
   uint32_t* sfrozen = sst + TILE_MAX_COLS;
   double* const cols = sm + TILE_HDR;
 
-  if (wid == 0) {
-    const uint32_t where = uint32_t(__cvta_generic_to_shared(ctl));
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(where) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
-  }
+  if (wid == 0) tm_alloc<512>(ctl);
   if (tid == 0) {
     ctl[1] = TILE_WARPS;
     ctl[2] = 0;
@@ -882,8 +878,7 @@ __global__ void __launch_bounds__(TILE_THREADS, 1) vert_tile_kernel(const KParam
     }
     __syncthreads();
   }
-  if (wid == 0)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tm_base));
+  if (wid == 0) tm_free<512>(tm_base);
 }
 
 }  // namespace gv
