@@ -743,10 +743,10 @@ __device__ inline double cell_adjoint_species(const ColCtx& c, const ColAdj& a, 
 #pragma unroll
     for (int e = 0; e < NS; ++e) pe[e] = (dt * c_k.kpair[e]) * pe[e];
 #pragma unroll
-    for (int s = 0; s < NS; ++s) {
-      mn[s] = c_k.mass[s] * ns[s];
-      vsol[s] = mn[s] * wv[s];
-    }
+    for (int s = 0; s < NS; ++s) mn[s] = c_k.mass[s] * ns[s];
+    const bool trace = friction_trace(ns, mn);
+#pragma unroll
+    for (int s = 0; s < NS; ++s) vsol[s] = mn[s] * wv[s];
     FrictionLdl ldl;
     ldl.factor(ns, mn, pe);
     ldl.eliminate(vsol);
@@ -811,6 +811,10 @@ __device__ inline double cell_adjoint_species(const ColCtx& c, const ColAdj& a, 
 #pragma unroll
     for (int s = 0; s < NS; ++s) wb[s] *= mn[s];
     Tb += ltb / T;
+    if (trace) {
+#pragma unroll
+      for (int s = 0; s < NS; ++s) ns[s] = exp_any(c.x(F_LNS + s, i));
+    }
   } else {
     __syncwarp();
     tm_get(kb, k0);

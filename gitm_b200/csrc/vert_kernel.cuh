@@ -551,6 +551,29 @@ struct FrictionLdl {
   }
 };
 
+// A row scaled by the species' mass density is no row of normal numbers for a
+// density below 1e-282, so for the solve a species of less than FRICTION_TRACE
+// counts as one of that density: its own row keeps its solution (both sides
+// scale with it), and in the other species' rows, whose diagonals are at least
+// their own M n, a coupling of 1e-42 FRICTION_TRACE is nothing.  True where one
+// of the densities was such a trace; a negative one or a NaN is not.
+constexpr double FRICTION_TRACE = 0x1p-900;
+template <bool WARP = false>
+__device__ __forceinline__ bool friction_trace(double (&ns)[NS], double (&mn)[NS]) {
+  bool any = false;
+#pragma unroll
+  for (int s = 0; s < NS; ++s) any = any || unsigned(__double2hiint(ns[s])) < 0x07b00000u;
+  if (m_any<WARP>(any)) {
+#pragma unroll
+    for (int s = 0; s < NS; ++s) {
+      const bool t = unsigned(__double2hiint(ns[s])) < 0x07b00000u;
+      ns[s] = t ? FRICTION_TRACE : ns[s];
+      mn[s] = t ? c_k.mass[s] * FRICTION_TRACE : mn[s];
+    }
+  }
+  return any;
+}
+
 // The friction solve in place of wv.  A non-finite density or temperature
 // takes the reference's row test, which sets GITM_ST_LU_SINGULAR in *st (when
 // st is given); the solve goes on, its results non-finite.  WARP: whole warps
@@ -582,10 +605,17 @@ __device__ __forceinline__ void friction_solve(double dt, const double (&ns)[NS]
   }
 #pragma unroll
   for (int e = 0; e < NS; ++e) pw[e] = (dt * c_k.kpair[e]) * pw[e];
+  double nf[NS], mf[NS];
 #pragma unroll
-  for (int r = 0; r < NS; ++r) wv[r] *= mn[r];
+  for (int s = 0; s < NS; ++s) {
+    nf[s] = ns[s];
+    mf[s] = mn[s];
+  }
+  friction_trace<WARP>(nf, mf);
+#pragma unroll
+  for (int r = 0; r < NS; ++r) wv[r] *= mf[r];
   FrictionLdl m;
-  m.factor(ns, mn, pw);
+  m.factor(nf, mf, pw);
   m.eliminate(wv);
   m.back(wv);
 }
