@@ -202,11 +202,15 @@ static cudaError_t plan_alloc(GitmVertPlan* P, T** p, size_t count) {
   return e;
 }
 
+// An error that is reported is also taken from the runtime's record, where the
+// check of a later call's launch would meet it again.
 #define CUDA_TRY(ctx, call)                                                              \
   do {                                                                                   \
     cudaError_t e_ = (call);                                                             \
-    if (e_ != cudaSuccess)                                                               \
+    if (e_ != cudaSuccess) {                                                             \
+      cudaGetLastError();                                                                \
       return set_err((ctx), GITM_ERR_CUDA, "%s failed: %s", #call, cudaGetErrorString(e_)); \
+    }                                                                                    \
   } while (0)
 
 // ------------------------------------------------------------------ constants
@@ -787,6 +791,7 @@ int gitm_vert_plan_wait(GitmVertPlan* P, void* stream, double timeout_s) {
     e = cudaEventQuery(ev);
     if (e == cudaSuccess) break;
     if (e != cudaErrorNotReady) break;
+    cudaGetLastError();
     e = cudaSuccess;
     const double el = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
     if (el >= timeout_s) {
@@ -1751,9 +1756,10 @@ extern "C" int gitm_vert_advance_fortran(GitmVertCtx* ctx, const GitmFortranStat
     }
     // cells in up to 8 parts, so that small calls fill the chip too
     const dim3 grid(unsigned((ncols + 255) / 256), unsigned(v.size()), 8);
-    fortran_copy_kernel<<<grid, 256>>>(d_maps + (dir ? in.size() : 0), base, dir, nLons, nLats, block_first, int(ncols));
-    const cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return set_err(ctx, GITM_ERR_CUDA, "fortran copy: %s", cudaGetErrorString(e));
+    const FMap* maps = d_maps + (dir ? in.size() : 0);
+    int cols = int(ncols), lons = nLons, lats = nLats, first = block_first;
+    void* args[] = {&maps, &base, &dir, &lons, &lats, &first, &cols};
+    CUDA_TRY(ctx, cudaLaunchKernel((const void*)fortran_copy_kernel, grid, dim3(256), args, 0, nullptr));
     return GITM_OK;
   };
   if (!rc && on_device) {

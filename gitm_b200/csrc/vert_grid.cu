@@ -95,8 +95,8 @@ cudaError_t grid_launch(int nAlts, int64_t gcols, const double* alt, const doubl
                         const double* inv_r, double* out, cudaStream_t stream) {
   if (gcols <= 0) return cudaSuccess;
   const dim3 grid(unsigned((gcols + GRID_THREADS - 1) / GRID_THREADS), unsigned(nAlts + 4));
-  grid_kernel<<<grid, GRID_THREADS, 0, stream>>>(nAlts, gcols, alt, grav, dalt_c, inv_r, out);
-  return cudaGetLastError();
+  void* args[] = {&nAlts, &gcols, &alt, &grav, &dalt_c, &inv_r, &out};
+  return cudaLaunchKernel((const void*)grid_kernel, grid, dim3(GRID_THREADS), args, 0, stream);
 }
 
 }  // namespace gv
