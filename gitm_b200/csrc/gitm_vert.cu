@@ -559,7 +559,7 @@ static int plan_common(GitmVertPlan* P, const double* const* alt, const double* 
                        const double* const* dalt, const double* const* invr, const int* gpc) {
   GitmVertCtx* ctx = P->ctx;
   // grid coefficients, formed on the device (vert_grid.cu); a member whose
-  // grid is in host memory has it copied behind the coefficients first
+  // grid the kernel cannot read in place has it copied behind the coefficients
   std::vector<size_t> goff(P->n_members), hoff(P->n_members, 0);
   std::vector<double> host_grids;
   size_t gtotal = 0;
@@ -572,7 +572,12 @@ static int plan_common(GitmVertPlan* P, const double* const* alt, const double* 
   for (int m = 0; m < P->n_members; ++m) {
     const double* src[4] = {alt[m], grav[m], dalt[m], invr[m]};
     bool device = true;
-    for (const double* p : src) device = device && is_device_ptr(p);
+    for (const double* p : src) {
+      cudaPointerAttributes a;
+      const cudaError_t e = cudaPointerGetAttributes(&a, p);
+      if (e != cudaSuccess) cudaGetLastError();
+      device = device && grid_in_place(p, e, a, ctx->device);
+    }
     if (device) continue;
     const int64_t per = int64_t(P->host_members[m].n_alts + 4) * (gpc[m] ? P->host_members[m].n_cols : 1);
     hoff[m] = gtotal + host_grids.size();
