@@ -13,6 +13,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <initializer_list>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -36,15 +37,18 @@ using namespace gv;
 // its allocations and frees took most of it: 0.8 of 0.93 ms at 2,592 columns,
 // where the step takes 0.14.  A context and its plans share one pool; it holds
 // at most kLimit bytes and gives everything back with the last of them.  A
-// block comes back only once the device has finished with it (plan_free and
+// block comes back only once the device has finished with it (give and
 // build_tiles synchronise first, as cudaFree did), so any stream may use it
-// next; the mutex makes it safe from several host threads.
+// next; where the device cannot be waited for (a stream is being captured), it
+// is set aside until a later wait has succeeded.  The mutex makes the pool safe
+// from several host threads.
 class DevPool {
  public:
   explicit DevPool(int device) : device_(device) {}
   ~DevPool() {
     int was = 0;
     const bool ok = cudaGetDevice(&was) == cudaSuccess && cudaSetDevice(device_) == cudaSuccess;
+    for (void* p : aside_) cudaFree(p);
     trim();
     if (ok) cudaSetDevice(was);
   }
@@ -71,11 +75,24 @@ class DevPool {
     if (e == cudaSuccess) size_[*p] = bytes;
     return e;
   }
-  // Waits for everything launched on the pool's device, as cudaFree does.
-  void drain() {
+  // Waits for everything launched on the pool's device, as cudaFree does, and
+  // takes back blocks of get() (or NULL) that only work launched so far uses.
+  void give(std::initializer_list<void*> blocks) {
+    std::vector<void*> done;
+    {
+      std::lock_guard<std::mutex> lock(mu_);
+      done.swap(aside_);
+    }
+    done.insert(done.end(), blocks.begin(), blocks.end());
     int was = 0;
     const bool ok = cudaGetDevice(&was) == cudaSuccess && cudaSetDevice(device_) == cudaSuccess;
-    cudaDeviceSynchronize();
+    if (cudaDeviceSynchronize() == cudaSuccess) {
+      for (void* p : done) put(p);
+    } else {
+      cudaGetLastError();
+      std::lock_guard<std::mutex> lock(mu_);
+      aside_.insert(aside_.end(), done.begin(), done.end());
+    }
     if (ok) cudaSetDevice(was);
   }
   // p: a block of get() that nothing on the device uses any more, or NULL
@@ -103,6 +120,7 @@ class DevPool {
   std::mutex mu_;
   std::multimap<size_t, void*> free_;
   std::map<void*, size_t> size_;  // blocks given out
+  std::vector<void*> aside_;      // given back, but perhaps still in use
   size_t held_ = 0;
 };
 
@@ -620,11 +638,8 @@ static int plan_common(GitmVertPlan* P, const double* const* alt, const double* 
 
 static void plan_free(GitmVertPlan* P) {
   if (!P) return;
-  P->pool->drain();  // what the plan launched, on any stream, is done with its memory
-  for (void* p : {(void*)P->d_adj_tiles, (void*)P->d_save_tiles, (void*)P->d_adj_states,
-                  (void*)P->d_bars, (void*)P->d_scratch, (void*)P->d_members, (void*)P->d_grid, (void*)P->d_status,
-                  (void*)P->d_tiles})
-    P->pool->put(p);
+  P->pool->give({P->d_adj_tiles, P->d_save_tiles, P->d_adj_states, P->d_bars, P->d_scratch, P->d_members, P->d_grid,
+                 P->d_status, P->d_tiles});
   delete P;
 }
 
@@ -1794,10 +1809,7 @@ extern "C" int gitm_vert_advance_fortran(GitmVertCtx* ctx, const GitmFortranStat
     }
     if (rc2) rc = rc2;
   }
-  if (d_maps) {
-    ctx->pool->drain();
-    ctx->pool->put(d_maps);
-  }
+  if (d_maps) ctx->pool->give({d_maps});
   ctx->params = saved;
   return rc;
 }
