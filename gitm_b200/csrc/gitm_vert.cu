@@ -25,6 +25,7 @@
 #include "vert_kernel.cuh"
 #include "vert_tile.cuh"
 #include "vert_adjoint.cuh"
+#include "vert_chunks.h"
 #include "vert_instances.h"
 #include "vert_hz.cuh"
 #include "vert_grid.cuh"
@@ -189,8 +190,7 @@ struct GitmVertPlan {
   GitmColumnAdjoint* d_bars = nullptr;
   // the saving step kernel (its own tiles and persistent grid)
   // tile ranges whose stage states a call without saved ones forms and
-  // reverses together, and their buffer
-  struct AdjChunk { int save0, save1, adj0, adj1; int64_t c0, n; };
+  // reverses together, and their buffer (of the first such call)
   std::vector<AdjChunk> adj_chunks;
   double* d_adj_states = nullptr;
   std::vector<Tile> save_tiles;
@@ -943,36 +943,28 @@ constexpr int kAdjThreads = ADJ_THREADS;
 
 // The tile ranges and the buffer of a call without saved states: about five
 // rounds of the adjoint kernel's grid at a time (2,960 columns of 50
-// altitudes, 157 MB), whole tiles of both kernels.
-static int adjoint_chunks(GitmVertPlan* P, int64_t columns) {
-  GitmVertCtx* ctx = P->ctx;
+// altitudes, 157 MB), or as many as there is memory for.  Formed by the first
+// such call; callers that keep the states themselves never need it.
+static int adjoint_chunks(GitmVertPlan* P) {
   if (!P->adj_chunks.empty()) return GITM_OK;
-  std::vector<GitmVertPlan::AdjChunk> out;
-  size_t s = 0, a = 0;
-  int64_t off = 0, most = 0;
-  for (int m = 0; m < P->n_members; ++m) {
-    const int64_t n_cols = P->host_members[m].n_cols;
-    if (n_cols == 0) continue;
-    const int64_t both = int64_t(P->save_tiles[s].nc) * P->adj_tiles[a].nc;  // a boundary of both tilings
-    const int64_t step = std::max<int64_t>(1, columns / both) * both;
-    for (int64_t c0 = 0; c0 < n_cols; c0 += step) {
-      const int64_t c1 = std::min(n_cols, c0 + step);
-      GitmVertPlan::AdjChunk ch{int(s), 0, int(a), 0, off + c0, c1 - c0};
-      while (s < P->save_tiles.size() && P->save_tiles[s].member == m && P->save_tiles[s].c0 < c1) ++s;
-      while (a < P->adj_tiles.size() && P->adj_tiles[a].member == m && P->adj_tiles[a].c0 < c1) ++a;
-      ch.save1 = int(s);
-      ch.adj1 = int(a);
-      most = std::max(most, ch.n);
-      out.push_back(ch);
+  GitmVertCtx* ctx = P->ctx;
+  std::vector<int64_t> n_cols;
+  for (const GitmColumnBatch& b : P->host_members) n_cols.push_back(b.n_cols);
+  int64_t columns = 5 * int64_t(P->adj_grid) * P->adj_tiles[0].nc, last = 0;
+  for (;;) {
+    std::vector<AdjChunk> cut = adjoint_cut(P->save_tiles, P->adj_tiles, n_cols, columns);
+    const int64_t most = adjoint_cut_largest(cut);
+    if (most != last &&
+        plan_alloc(P, &P->d_adj_states, size_t(ADJ_NSTATE) * most * P->adj_per_max) == cudaSuccess) {
+      P->adj_chunks = std::move(cut);
+      return GITM_OK;
     }
-    off += n_cols;
-  }
-  if (plan_alloc(P, &P->d_adj_states, size_t(ADJ_NSTATE) * most * P->adj_per_max) != cudaSuccess) {
     cudaGetLastError();
-    return set_err(ctx, GITM_ERR_NOMEM, "adjoint: cannot allocate the stage states of %lld columns", (long long)most);
+    if (columns <= 1)
+      return set_err(ctx, GITM_ERR_NOMEM, "adjoint: cannot allocate the stage states of %lld columns", (long long)most);
+    last = most;
+    columns /= 2;
   }
-  P->adj_chunks = std::move(out);
-  return GITM_OK;
 }
 
 // Tiles and persistent grid of the adjoint kernel for the plan.
@@ -1045,8 +1037,6 @@ static int adjoint_prepare(GitmVertPlan* P) {
   CUDA_TRY(ctx, plan_alloc(P, &P->d_save_tiles, P->save_tiles.size()));
   CUDA_TRY(ctx, cudaMemcpy(P->d_save_tiles, P->save_tiles.data(), P->save_tiles.size() * sizeof(Tile),
                            cudaMemcpyHostToDevice));
-  const int rc = adjoint_chunks(P, 5 * int64_t(P->adj_grid) * P->adj_tiles[0].nc);
-  if (rc) return rc;
   P->adj_ready = true;
   return GITM_OK;
 }
@@ -1154,7 +1144,9 @@ extern "C" int gitm_vert_plan_adjoint(GitmVertPlan* P, const GitmColumnAdjoint* 
     return GITM_OK;
   };
   if (saved_states) return launch(0, int(P->adj_tiles.size()), saved_states, 0, P->n_cols_total);
-  for (const GitmVertPlan::AdjChunk& ch : P->adj_chunks) {
+  rc = adjoint_chunks(P);
+  if (rc) return rc;
+  for (const AdjChunk& ch : P->adj_chunks) {
     rc = launch_saving(P, dt, ch.save0, ch.save1, P->d_adj_states, ch.c0, ch.n, false, st);
     if (!rc) rc = launch(ch.adj0, ch.adj1, P->d_adj_states, ch.c0, ch.n);
     if (rc) return rc;
