@@ -26,7 +26,7 @@ SOURCES = ["gitm_vert.cu", "vert_adjoint.cu", "hz_kernel.cu", "vert_grid.cu"]
 # the grid coefficients round as the reference's, which uses no fused multiply-add
 EXTRA_FLAGS = {"vert_grid.cu": ["-fmad=false"]}
 DEPS = ["gitm_vert.cu", "vert_adjoint.cu", "hz_kernel.cu", "vert_instance.cu", "vert_instances.h", "vert_kernel.cuh",
-        "vert_ausm.cuh", "vert_adjoint.cuh", "vert_common.cuh", "vert_hz.cuh", "vert_math.cuh", "vert_tile.cu", "vert_tile.cuh", "vert_tmem.cuh", "vert_chunks.h",
+        "vert_ausm.cuh", "vert_adjoint.cuh", "vert_common.cuh", "vert_hz.cuh", "vert_math.cuh", "vert_tile.cu", "vert_tile.cuh", "vert_tmem.cuh", "vert_chunks.h", "dev_pool.h",
         "vert_grid.cu", "vert_grid.cuh"]
 
 NVCC_FLAGS = [

@@ -13,14 +13,12 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
-#include <initializer_list>
-#include <map>
 #include <memory>
-#include <mutex>
 #include <string>
 #include <thread>
 #include <vector>
 
+#include "dev_pool.h"
 #include "vert_common.cuh"
 #include "vert_kernel.cuh"
 #include "vert_tile.cuh"
@@ -31,99 +29,6 @@
 #include "vert_grid.cuh"
 
 using namespace gv;
-
-// ------------------------------------------------------------------ memory
-// Device blocks of plans that are gone, for the next plan.  The one-shot calls
-// (advance_native, advance_fortran, the torch op) build a plan per call, and
-// its allocations and frees took most of it: 0.8 of 0.93 ms at 2,592 columns,
-// where the step takes 0.14.  A context and its plans share one pool; it holds
-// at most kLimit bytes and gives everything back with the last of them.  A
-// block comes back only once the device has finished with it (give and
-// build_tiles synchronise first, as cudaFree did), so any stream may use it
-// next; where the device cannot be waited for (a stream is being captured), it
-// is set aside until a later wait has succeeded.  The mutex makes the pool safe
-// from several host threads.
-class DevPool {
- public:
-  explicit DevPool(int device) : device_(device) {}
-  ~DevPool() {
-    int was = 0;
-    const bool ok = cudaGetDevice(&was) == cudaSuccess && cudaSetDevice(device_) == cudaSuccess;
-    for (void* p : aside_) cudaFree(p);
-    trim();
-    if (ok) cudaSetDevice(was);
-  }
-  DevPool(const DevPool&) = delete;
-  DevPool& operator=(const DevPool&) = delete;
-
-  cudaError_t get(void** p, size_t bytes) {
-    bytes = (std::max<size_t>(bytes, 1) + 511) & ~size_t(511);
-    std::lock_guard<std::mutex> lock(mu_);
-    auto it = free_.lower_bound(bytes);
-    if (it != free_.end() && it->first <= std::max(2 * bytes, size_t(64) << 10)) {
-      *p = it->second;
-      held_ -= it->first;
-      size_[*p] = it->first;
-      free_.erase(it);
-      return cudaSuccess;
-    }
-    cudaError_t e = cudaMalloc(p, bytes);
-    if (e == cudaErrorMemoryAllocation) {
-      cudaGetLastError();
-      trim();
-      e = cudaMalloc(p, bytes);
-    }
-    if (e == cudaSuccess) size_[*p] = bytes;
-    return e;
-  }
-  // Waits for everything launched on the pool's device, as cudaFree does, and
-  // takes back blocks of get() (or NULL) that only work launched so far uses.
-  void give(std::initializer_list<void*> blocks) {
-    std::vector<void*> done;
-    {
-      std::lock_guard<std::mutex> lock(mu_);
-      done.swap(aside_);
-    }
-    done.insert(done.end(), blocks.begin(), blocks.end());
-    int was = 0;
-    const bool ok = cudaGetDevice(&was) == cudaSuccess && cudaSetDevice(device_) == cudaSuccess;
-    if (cudaDeviceSynchronize() == cudaSuccess) {
-      for (void* p : done) put(p);
-    } else {
-      cudaGetLastError();
-      std::lock_guard<std::mutex> lock(mu_);
-      aside_.insert(aside_.end(), done.begin(), done.end());
-    }
-    if (ok) cudaSetDevice(was);
-  }
-  // p: a block of get() that nothing on the device uses any more, or NULL
-  void put(void* p) {
-    if (!p) return;
-    std::lock_guard<std::mutex> lock(mu_);
-    const size_t bytes = size_[p];
-    size_.erase(p);
-    if (held_ + bytes <= kLimit) {
-      free_.emplace(bytes, p);
-      held_ += bytes;
-    } else {
-      cudaFree(p);
-    }
-  }
-
- private:
-  static constexpr size_t kLimit = size_t(256) << 20;
-  void trim() {
-    for (auto& b : free_) cudaFree(b.second);
-    free_.clear();
-    held_ = 0;
-  }
-  const int device_;
-  std::mutex mu_;
-  std::multimap<size_t, void*> free_;
-  std::map<void*, size_t> size_;  // blocks given out
-  std::vector<void*> aside_;      // given back, but perhaps still in use
-  size_t held_ = 0;
-};
 
 // ------------------------------------------------------------------ context
 struct GitmVertCtx {
@@ -216,6 +121,15 @@ template <class T>
 static cudaError_t plan_alloc(GitmVertPlan* P, T** p, size_t count) {
   void* v = nullptr;
   const cudaError_t e = P->pool->get(&v, count * sizeof(T));
+  *p = (e == cudaSuccess) ? static_cast<T*>(v) : nullptr;
+  return e;
+}
+
+// A context's own device memory.
+template <class T>
+static cudaError_t ctx_alloc(GitmVertCtx* ctx, T** p, size_t count) {
+  void* v = nullptr;
+  const cudaError_t e = ctx->pool->outside(&v, count * sizeof(T));
   *p = (e == cudaSuccess) ? static_cast<T*>(v) : nullptr;
   return e;
 }
@@ -844,7 +758,7 @@ static int snapshot(GitmVertPlan* P, std::vector<std::pair<double*, double*>>& b
       for (auto& f : fs) {
         if (!f.p) continue;
         double* cp = nullptr;
-        CUDA_TRY(ctx, cudaMalloc(&cp, cells * f.k * sizeof(double)));
+        CUDA_TRY(ctx, ctx_alloc(ctx, &cp, cells * f.k));
         CUDA_TRY(ctx, cudaMemcpy(cp, f.p, cells * f.k * sizeof(double), cudaMemcpyDeviceToDevice));
         bk.push_back({f.p, cp});
       }
@@ -1161,7 +1075,7 @@ static int arena_reserve(GitmVertCtx* ctx, size_t bytes) {
   cudaFree(ctx->arena);
   ctx->arena = nullptr;
   ctx->arena_bytes = 0;
-  if (cudaMalloc(&ctx->arena, bytes) != cudaSuccess) {
+  if (ctx_alloc(ctx, &ctx->arena, bytes) != cudaSuccess) {
     cudaGetLastError();
     return set_err(ctx, GITM_ERR_NOMEM, "cannot allocate %zu bytes of device staging", bytes);
   }
@@ -1550,7 +1464,7 @@ extern "C" int gitm_vert_cfl_dt(GitmVertCtx* ctx, const GitmColumnBatch* members
                                 double dt_in, double dt_end, double* dt_out) {
   if (!ctx || !dt_out || (n_members > 0 && !members)) return set_err(ctx, GITM_ERR_ARG, "bad arguments");
   CUDA_TRY(ctx, cudaSetDevice(ctx->device));
-  if (!ctx->d_scalar) CUDA_TRY(ctx, cudaMalloc(&ctx->d_scalar, sizeof(double)));
+  if (!ctx->d_scalar) CUDA_TRY(ctx, ctx_alloc(ctx, &ctx->d_scalar, 1));
   // all ones: above every positive double, so an untouched word means no step
   CUDA_TRY(ctx, cudaMemsetAsync(ctx->d_scalar, 0xff, sizeof(double)));
   for (int m = 0; m < n_members; ++m) {
@@ -2019,7 +1933,7 @@ extern "C" int gitm_hz_advance(GitmVertCtx* ctx, const GitmHzParams* params, con
     cudaFree(ctx->hz_status);
     ctx->hz_status = nullptr;
     ctx->hz_status_n = 0;
-    if (cudaMalloc(&ctx->hz_status, size_t(b.n_blocks) * sizeof(uint32_t)) != cudaSuccess) {
+    if (ctx_alloc(ctx, &ctx->hz_status, size_t(b.n_blocks)) != cudaSuccess) {
       cudaGetLastError();
       return set_err(ctx, GITM_ERR_NOMEM, "cannot allocate the block status words");
     }
@@ -2057,7 +1971,7 @@ extern "C" int gitm_hz_exchange(GitmVertCtx* ctx, const GitmHzExchange* x, void*
     cudaFree(ctx->hz_status);
     ctx->hz_status = nullptr;
     ctx->hz_status_n = 0;
-    if (cudaMalloc(&ctx->hz_status, size_t(nb) * sizeof(uint32_t)) != cudaSuccess) {
+    if (ctx_alloc(ctx, &ctx->hz_status, size_t(nb)) != cudaSuccess) {
       cudaGetLastError();
       return set_err(ctx, GITM_ERR_NOMEM, "cannot allocate the block status words");
     }
