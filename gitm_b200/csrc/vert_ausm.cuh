@@ -164,7 +164,11 @@ __device__ __forceinline__ void exp_faces(const Faces& t, double base, double (&
 }
 
 // AUSM+-up numerical velocity (Mach split, pressure diffusion) at one face
-// and the species flux pair; (:1660-1937).  ics = 1 / cs.
+// and the species flux pair; (:1660-1937).  ics = 1 / cs; kp = LiouKpS times
+// MPRESS_SCALE, which with the mean density's keeps the pressure diffusion's
+// denominator a normal number for a species of hardly any density (both
+// products are exact).
+constexpr double MPRESS_SCALE = 0x1p200;
 __device__ __forceinline__ void species_face_flux(double rl, double rr, double pl, double pr, double hl,
                                                   double hr, double wl, double wr, double cs, double ics, double kp,
                                                   double ku, double dzdt, bool subtract, double& nv,
@@ -182,7 +186,7 @@ __device__ __forceinline__ void species_face_flux(double rl, double rr, double p
   // sound speed and less).  For |M| >= 1: (M + |M|) / 2 and (M - |M|) / 2.
   const double FL = (fabs(Ml) >= 1.0) ? 0.5 * (Ml + fabs(Ml)) - 0.375 : fma(0.125 * Ml2, Ml2, 0.5 * Ml);
   const double FR = (fabs(Mr) >= 1.0) ? 0.5 * (Mr - fabs(Mr)) + 0.375 : fma(-0.125 * Mr2, Mr2, 0.5 * Mr);
-  const double meanrho = 0.5 * (rl + rr);
+  const double meanrho = (0.5 * MPRESS_SCALE) * (rl + rr);
   const double dp = subtract ? ((pr - hr) - (pl - hl)) : (pr - pl);
   const double MPress = kp * fmax(1.0 - M2Bar, 0.0) * dp * rcp_nr(meanrho * cs * (FA * cs + 1.0 * dzdt));
   nv = cs * (FL + FR - MPress);
@@ -345,7 +349,7 @@ __device__ __forceinline__ void ausm_cell(ColCtx c, int i, const GitmVertParams&
   // ---- pass 2: species fluxes, continuity and species momentum (:844-900)
   const double AP = c.ga(GA_AP, i), AM = c.ga(GA_AM, i), Vol = c.ga(GA_VOL, i);
   const double dAltC = c.ga(GA_DALTC, i);
-  const double kp = c.ga(GA_KP, i), ku = c.ga(GA_KU, i);
+  const double kp = MPRESS_SCALE * c.ga(GA_KP, i), ku = c.ga(GA_KU, i);
   const double dzdt = dAltC / dtk;
   const double hz = dtk * (VN * VN + VE * VE) * invr;
   const double iCSM = rcp_nr(CSM), iCSP = rcp_nr(CSP), iVol = rcp_nr(Vol), idAltC = rcp_nr(dAltC);
