@@ -32,6 +32,7 @@
 #include "../../include/gitm_hz.h"
 #include "vert_common.cuh"
 #include "vert_hz.cuh"
+#include "vert_math.cuh"
 
 namespace gv {
 
@@ -82,17 +83,6 @@ __host__ __device__ inline HzLayout hz_layout(int nLons, int nLats, int batch, b
   return L;
 }
 
-// ModLimiter.f90:16-36 without branches (limiter_mc of the vertical step).
-__device__ __forceinline__ double hz_limiter(double u, double d, double beta) {
-  const double au = fabs(u), ad = fabs(d);
-  const double t = beta * (au < ad ? au : ad);
-  const double s = (u + d) * 0.5, as = fabs(s);
-  const double m = t < as ? t : as;
-  const bool same = (__double2hiint(u) ^ __double2hiint(d)) >= 0;
-  const int hi = __double2hiint(m) | (__double2hiint(u) & int(0x80000000u));
-  return same ? __hiloint2double(hi, __double2loint(m)) : 0.0;
-}
-
 // The limited slopes of one line (calc_facevalues_lons / _lats): cells 0 ..
 // n+1 of values V and inverse face distances IF, both with stride s (index 0
 // = cell -1), to d with stride sd.  4th-order differences, with the 2nd-order
@@ -108,13 +98,13 @@ __device__ __forceinline__ void hz_slopes(const double* V, const double* IF, dou
     // between cells q and q+1
     const double vq = V[(q + 3) * s];
     const double up = (IF[(q + 2) * s] * 2) * (F1 * (vp - v0) - F2 * (vq - vm));
-    d[q * sd] = hz_limiter(up, dn, beta);
+    d[q * sd] = limiter_mc(up, dn, beta);
     dn = up;
     vm = v0;
     v0 = vp;
     vp = vq;
   }
-  d[(n + 1) * sd] = hz_limiter((vp - v0) * IF[(n + 3) * s], dn, beta);
+  d[(n + 1) * sd] = limiter_mc((vp - v0) * IF[(n + 3) * s], dn, beta);
 }
 
 // A cell's faces along one direction: halves of the face widths, the

@@ -112,23 +112,6 @@ __device__ __forceinline__ bool in_pcells(int i, int nAlts) {
 
 __device__ __forceinline__ bool photochemical(int s) { return s == 3 || s == 4; }  // N(4S), NO
 
-// ModLimiter.f90:16-36, without branches: on same-sign slopes the smallest
-// magnitude of beta u, beta d and (u + d) / 2 carries the common sign (the
-// reference's min of the three when both are positive and max when both are
-// negative, the same values since negation is exact and rounding monotonic:
-// min(beta |u|, beta |d|) = beta min(|u|, |d|)); 0 otherwise.  Selects on
-// plain comparisons and the sign bits: fmin and the four comparisons with
-// zero took about twice the instructions.
-__device__ __forceinline__ double limiter_mc(double u, double d, double beta) {
-  const double au = fabs(u), ad = fabs(d);
-  const double t = beta * (au < ad ? au : ad);
-  const double s = (u + d) * 0.5, as = fabs(s);
-  const double m = t < as ? t : as;
-  const bool same = (__double2hiint(u) ^ __double2hiint(d)) >= 0;  // a zero among them makes m zero
-  const int hi = __double2hiint(m) | (__double2hiint(u) & int(0x80000000u));
-  return same ? __hiloint2double(hi, __double2loint(m)) : 0.0;
-}
-
 struct ColCtx {
   double* col;
   Layout L;
