@@ -744,13 +744,18 @@ __device__ inline double cell_adjoint_species(const ColCtx& c, const ColAdj& a, 
     for (int e = 0; e < NS; ++e) pe[e] = (dt * c_k.kpair[e]) * pe[e];
 #pragma unroll
     for (int s = 0; s < NS; ++s) mn[s] = c_k.mass[s] * ns[s];
-    const bool trace = friction_trace(ns, mn);
+    const double shift = friction_range(ns, mn, pe);
 #pragma unroll
     for (int s = 0; s < NS; ++s) vsol[s] = mn[s] * wv[s];
     FrictionLdl ldl;
     ldl.factor(ns, mn, pe);
     ldl.eliminate(vsol);
     ldl.back(vsol);
+    auto densities = [&] {  // the cell's own again
+#pragma unroll
+      for (int s = 0; s < NS; ++s) ns[s] = exp_any(c.x(F_LNS + s, i));
+    };
+    if (shift != 0.0) densities();
     // clamp, bulk wind and their reverse
     __syncwarp();
     tm_get(kb, k0);
@@ -793,6 +798,14 @@ __device__ inline double cell_adjoint_species(const ColCtx& c, const ColAdj& a, 
     for (int s = 0; s < NS; ++s) wb[s] = vb[s];
     ldl.forward(wb);
     ldl.back(wb);
+    if (shift != 0.0) {
+      // a density times y is the same at either scale
+#pragma unroll
+      for (int s = 0; s < NS; ++s) {
+        pe[s] *= shift;
+        ns[s] = mn[s] * c_k.inv_mass[s];
+      }
+    }
     // each pair (r, q) through its coefficient P = dt kpair T^(1-e), with y:
     // n_q takes P n_r y_r (v_q - v_r), n_r takes P n_q y_q (v_r - v_q), and log T
     // (1 - e) n_r n_q of both
@@ -810,11 +823,8 @@ __device__ inline double cell_adjoint_species(const ColCtx& c, const ColAdj& a, 
       }
 #pragma unroll
     for (int s = 0; s < NS; ++s) wb[s] *= mn[s];
-    Tb += ltb / T;
-    if (trace) {
-#pragma unroll
-      for (int s = 0; s < NS; ++s) ns[s] = exp_any(c.x(F_LNS + s, i));
-    }
+    Tb += (shift != 0.0 ? ltb / shift : ltb) / T;
+    if (shift != 0.0) densities();
   } else {
     __syncwarp();
     tm_get(kb, k0);

@@ -168,7 +168,7 @@ __device__ __forceinline__ void exp_faces(const Faces& t, double base, double (&
 // MPRESS_SCALE, which with the mean density's keeps the pressure diffusion's
 // denominator a normal number for a species of hardly any density (both
 // products are exact).
-constexpr double MPRESS_SCALE = 0x1p200;
+constexpr double MPRESS_SCALE = 0x1p64;
 __device__ __forceinline__ void species_face_flux(double rl, double rr, double pl, double pr, double hl,
                                                   double hr, double wl, double wr, double cs, double ics, double kp,
                                                   double ku, double dzdt, bool subtract, double& nv,

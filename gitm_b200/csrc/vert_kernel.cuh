@@ -545,27 +545,41 @@ struct FrictionLdl {
   }
 };
 
-// A row scaled by the species' mass density is no row of normal numbers for a
-// density below 1e-282, so for the solve a species of less than FRICTION_TRACE
-// counts as one of that density: its own row keeps its solution (both sides
-// scale with it), and in the other species' rows, whose diagonals are at least
-// their own M n, a coupling of 1e-42 FRICTION_TRACE is nothing.  True where one
-// of the densities was such a trace; a negative one or a NaN is not.
-constexpr double FRICTION_TRACE = 0x1p-900;
+// The solve's numbers are products of two densities, or of one with its mass.
+// For densities from 2^-700 to 2^500 they are normal; others, in any species,
+// take this way first.
+//
+// Below: a species of less than 2^-700 counts as one of that density.  Its own
+// row keeps its solution (both sides scale with it), and in the other species'
+// rows, whose diagonals are at least their own M n, a coupling of 1e-17 of that
+// density is nothing.  Above: the densities are divided by the power of two
+// that takes the largest to about 2^100, and the pair coefficients multiplied
+// by it, which scales the whole system; what falls below 2^-700 then is nothing
+// beside the largest.
+//
+// Returns 0 where the densities were in range, else the factor they were
+// multiplied by.  A negative density, an infinity or a NaN stays one.
 template <bool WARP = false>
-__device__ __forceinline__ bool friction_trace(double (&ns)[NS], double (&mn)[NS]) {
-  bool any = false;
+__device__ __forceinline__ double friction_range(double (&ns)[NS], double (&mn)[NS], double (&pe)[NS]) {
+  bool odd = false;
 #pragma unroll
-  for (int s = 0; s < NS; ++s) any = any || unsigned(__double2hiint(ns[s])) < 0x07b00000u;
-  if (m_any<WARP>(any)) {
+  for (int s = 0; s < NS; ++s) odd = odd || unsigned(__double2hiint(ns[s]) - 0x14300000) >= 0x5f300000u - 0x14300000u;
+  if (!m_any<WARP>(odd)) return 0.0;
+  double top = 0.0;
 #pragma unroll
-    for (int s = 0; s < NS; ++s) {
-      const bool t = unsigned(__double2hiint(ns[s])) < 0x07b00000u;
-      ns[s] = t ? FRICTION_TRACE : ns[s];
-      mn[s] = t ? c_k.mass[s] * FRICTION_TRACE : mn[s];
-    }
+  for (int s = 0; s < NS; ++s) top = fabs(ns[s]) > top ? fabs(ns[s]) : top;
+  const int e = (__double2hiint(top) >> 20) - 1023;
+  const int shift = e >= 500 ? e - 100 : 0;
+  const double f = __hiloint2double((1023 - shift) << 20, 0), g = __hiloint2double((1023 + shift) << 20, 0);
+#pragma unroll
+  for (int s = 0; s < NS; ++s) {
+    const double n = ns[s] * f;
+    const bool trace = unsigned(__double2hiint(n)) < 0x14300000u;  // positive and below 2^-700
+    ns[s] = trace ? 0x1p-700 : n;
+    mn[s] = trace ? c_k.mass[s] * 0x1p-700 : mn[s] * f;
+    pe[s] *= g;
   }
-  return any;
+  return odd ? f : 0.0;
 }
 
 // The friction solve in place of wv.  A non-finite density or temperature
@@ -605,7 +619,7 @@ __device__ __forceinline__ void friction_solve(double dt, const double (&ns)[NS]
     nf[s] = ns[s];
     mf[s] = mn[s];
   }
-  friction_trace<WARP>(nf, mf);
+  friction_range<WARP>(nf, mf, pw);
 #pragma unroll
   for (int r = 0; r < NS; ++r) wv[r] *= mf[r];
   FrictionLdl m;
