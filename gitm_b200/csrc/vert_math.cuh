@@ -1,21 +1,23 @@
 // vert_math.cuh -- FP64 exp, log and reciprocal for the stage kernels.
 //
 // What bounds a stage is the number of instructions its warps issue and the
-// latency of their FP64 chains.  CUDA's exp is 15 FP64 instructions among 49
-// (log: 30 of 81; their range tests, special cases and literal constants are
-// the rest), and ends in a branch, so the calls of a loop over species run
-// one after the other.  The batches here run N arguments side by side with
+// latency of their FP64 chains, and the calls of CUDA's exp and log in a loop
+// over species run one after the other: seven logarithms take one warp 1,900
+// cycles, in a batch 840.  The batches here run N arguments side by side with
 // one range test for all: 18 instructions per exp (15 FP64), 32 per log (23),
 // 5 per reciprocal.
 //
-// Written from the mathematics.  The range reduction is Cody and Waite's
-// (Software Manual for the Elementary Functions, 1980: ln 2 in two parts),
-// the polynomials are Chebyshev interpolants of (e^r - 1 - r) / r^2 on
-// |r| <= 0.347 (truncation 1.7e-17 relative) and of the atanh series on the
-// mantissas of [sqrt(1/2), sqrt(2)) (4.7e-18), the reciprocal refines PTX's
-// documented rcp.approx.ftz.f64 with Newton-Raphson steps.  Error against
-// the exact value: at most 0.94 ulp (exp), 0.96 ulp (log), 1 ulp
-// (reciprocal); tests/test_math.py, which compiles the header as plain C++.
+// Written from the mathematics and published methods.  exp's range reduction
+// is Cody and Waite's (Software Manual for the Elementary Functions, 1980:
+// ln 2 in two parts).  log's reduction to mantissas in [sqrt(1/2), sqrt(2)) by
+// an offset of the exponent field, and the arrangement f - s (f - z p) that
+// keeps f's bits, are those of FreeBSD's msun (e_log.c, from Sun's fdlibm; musl
+// has them from there).  The polynomials are Chebyshev interpolants of (e^r - 1
+// - r) / r^2 on |r| <= 0.347 (truncation 1.7e-17 relative) and of the atanh
+// series on those mantissas (4.7e-18), computed for this file; the reciprocal
+// refines PTX's documented rcp.approx.ftz.f64 with Newton-Raphson steps.  Error
+// against the exact value, on the device and as plain C++: below 1 ulp (exp,
+// log, reciprocal); tests/test_gpu_math.py and tests/test_math.py.
 #pragma once
 
 #include <cstdint>
@@ -60,16 +62,15 @@ GV_MATH double m_make(int hi, int lo) {
   return x;
 }
 GV_MATH double m_fma(double a, double b, double c) { return std::fma(a, b, c); }
-// a seed of the documented accuracy (23 bits) where there is no GPU
+// a seed of the documented accuracy (20 bits) where there is no GPU
 GV_MATH double rcp_seed(double a) {
   const double r = 1.0 / a;
-  return m_make(m_hi(r), m_lo(r) & int(0xc0000000u));
+  return m_make(m_hi(r), 0);
 }
 #endif
 
 // The constants are read from constant memory, where an FP64 instruction
-// takes them as an operand: as literals each costs two moves and a register
-// pair.
+// takes them as an operand.
 #ifdef __CUDACC__
 static __constant__ double
 #else
