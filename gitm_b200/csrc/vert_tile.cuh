@@ -521,6 +521,11 @@ __global__ void __launch_bounds__(TILE_THREADS, 1) vert_tile_kernel(const KParam
         }
       }
     };
+    const bool dry = SAVE && kp.no_store != 0;
+    // MeanMajorMass of the last step, where it is formed (only its TempUnit is kept)
+    auto put_mmm = [&](int g, int cl, double mmm) {
+      if (b.mean_major_mass && !dry) b.mean_major_mass[gidx(0, g, cl)] = mmm;
+    };
     // the tasks of phase P
     const int ninner = nA - 4;  // cells 3 .. nAlts-2
     const int nrun = max(1, (ninner + 8) / 16);
@@ -582,6 +587,7 @@ __global__ void __launch_bounds__(TILE_THREADS, 1) vert_tile_kernel(const KParam
         // calc_pressure.f90:17-21,56-83; calc_rates.Earth.f90:34-50; calc_timestep.f90:114-118
         tile_producers(nd, ww, temperature, gamma, mmm, tu, cmx);
         if (!(g >= 1 && g <= nA + 2)) cmx = 0.0;
+        if (kp.n_steps == 1) put_mmm(g, cl, mmm);
       } else {
         gamma = b.gamma[gidx(0, g, cl)];
         mmm = b.mean_major_mass[gidx(0, g, cl)];
@@ -726,6 +732,7 @@ __global__ void __launch_bounds__(TILE_THREADS, 1) vert_tile_kernel(const KParam
               c.gm(ri) = gamma;
               c.cm(ri) = (ri >= 0 && ri <= nA + 1) ? cmx : 0.0;
               c.tu(ri) = tu;
+              if (step == kp.n_steps - 2) put_mmm(ri + 1, rcl, mmm);
               if (ri == -1) c.sc(SC_MMM_M1) = mmm;
               if (ri == 0) c.sc(SC_MMM_0) = mmm;
             }
@@ -811,14 +818,12 @@ __global__ void __launch_bounds__(TILE_THREADS, 1) vert_tile_kernel(const KParam
 
     // ---------------------------------------------------------- store
     // scatter, advance_vertical.f90:163-217
-    const bool dry = SAVE && kp.no_store != 0;
     for (int w = tid; w < nc * G && !dry; w += TILE_THREADS) {
       const int g = w / nc, cl = w - g * nc, i = g - 1;
       ColCtx c = ctx(cl);
       if (prm.compute_coefficients) {
         // the coefficients the last step ran with
         if (b.gamma) b.gamma[gidx(0, g, cl)] = c.gm(i);
-        if (b.mean_major_mass) b.mean_major_mass[gidx(0, g, cl)] = c.tu(i) * KB;
         if (b.temp_unit) b.temp_unit[gidx(0, g, cl)] = c.tu(i);
         if (b.cmax && g >= 1 && g <= nA + 2) b.cmax[gidx(0, g, cl)] = c.cm(i);
       }
