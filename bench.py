@@ -218,14 +218,23 @@ def opcount(n_alts: int, solver: str = "rusanov") -> float:
     return float(d[solver][str(n_alts)]["flop_eq_per_column_step"])
 
 
-def profile_traffic():
-    """DRAM bytes per column and launch of the step kernel (the state is read
-    and written once per launch, whatever the steps per launch) from the
-    committed ncu summary (profiles/vert_step_kernel_globe1deg.md), or None."""
+def step_kernel(threads: int, solver: str) -> str:
+    """The kernel behind a launch shape of a GITM-array plan."""
+    return "vert_tile_kernel" if solver == "rusanov" and threads == 512 else "vert_step_kernel"
+
+
+def profile_traffic(kernel: str = "vert_step_kernel"):
+    """DRAM bytes per column and launch of a kernel's 512-thread shape (the
+    state is read and written once per launch, whatever the steps per launch)
+    from the committed ncu summary (profiles/vert_step_kernel_globe1deg.md:
+    the tile kernel, and the step kernel that had the shape before it), or
+    None."""
     p = os.path.join(ROOT, "profiles", "vert_step_kernel_globe1deg.md")
     if not os.path.exists(p):
         return None
-    m = re.search(r"dram_bytes_per_column_per_launch:\s*([0-9.eE+]+)", open(p).read())
+    key = {"vert_step_kernel": "dram_bytes_per_column_per_launch",
+           "vert_tile_kernel": "tile_kernel_bytes_per_column_per_launch"}[kernel]
+    m = re.search(rf"^{key}:\s*([0-9.eE+]+)", open(p).read(), re.M)
     return float(m.group(1)) if m else None
 
 
@@ -508,14 +517,15 @@ def run_ours(args):
             pass
         bytes_cs = algorithmic_bytes_per_column_step(args.n_alts) / max(1, cfg.steps_per_launch)
         achieved = flops_cs * cs_launch / t_launch / 1e12
-        traffic = profile_traffic() if args.solver == "rusanov" else None
+        kernel = step_kernel(cfg.threads, args.solver)
+        traffic = profile_traffic(kernel) if kernel == "vert_tile_kernel" else None
         roof = {"bound": "fp64", "achieved": achieved, "peak": fp64_peak, "unit": "TFLOP/s",
                 "frac": achieved / fp64_peak,
                 "traffic": None if traffic is None else traffic * n_cols,
                 "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one launch of the "
                                   "2 deg globe (profiles/vert_step_kernel_globe1deg.md), per column and "
                                   "launch, times the columns of a launch",
-                "kernel": "vert_step_kernel",
+                "kernel": kernel,
                 "peak_source": "FP64 DGEMM (cuBLAS via torch.matmul 8192^3) measured in this run "
                                "(MEASURED_PEAKS.json has no FP64 figure)",
                 "flops_per_column_step": flops_cs,
