@@ -1751,7 +1751,7 @@ static __device__ __align__(256) double g_noalloc_scratch[kNoAllocDoubles];
 
 
 // Builds the member descriptor, the grid coefficients of the member's
-// shared altitude grid (the formulas of grid_coefs above) and the tile list
+// shared altitude grid (the formulas of vert_grid.cu) and the tile list
 // in the scratch.  One CTA.
 __global__ void noalloc_setup_kernel(GitmColumnBatch b, int nc, int n_tiles, double* base) {
   DevMember* dmem = reinterpret_cast<DevMember*>(base);

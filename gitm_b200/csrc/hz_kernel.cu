@@ -23,8 +23,10 @@
 // What bounds it is the FP64 pipe and the latency of its chains.  With one
 // thread per cell and every slope formed by each of the three cells that read
 // it (486 per field of a 9 x 9 plane instead of 198), 12 warps ran per SM at
-// 168 registers, spilling, and a 2 degree globe (10,000 planes of 9 x 9) took
-// 3.11 ms; with the slopes shared and five fields per thread 1.31 ms.
+// 168 registers, and a 2 degree globe (10,000 planes of 9 x 9) took 3.11 ms;
+// with the slopes shared and five fields per thread 1.32 ms.  Both spill: the
+// instance of two CTAs of 12 warps, at 80 registers, keeps part of a thread's
+// values in local memory.
 #include <cuda_runtime.h>
 
 #include <cstdint>

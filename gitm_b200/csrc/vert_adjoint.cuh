@@ -26,8 +26,8 @@
 //
 // What bounds it: chains and the arrival of instructions at 8 warps per SM
 // (255 registers a thread); the FP64 pipe is a quarter busy.  A 2.5 degree
-// rollout (4 steps, checkpoints every 2, 10,368 columns) 16.3 -> 13.9 ms, one
-// step forward and backward of 2,592 columns 1.30 -> 1.13 ms with tensor
+// rollout (4 steps, checkpoints every 2, 10,368 columns) 16.3 -> 14.1 ms, one
+// step forward and backward of 2,592 columns 1.30 -> 1.14 ms with tensor
 // memory for global scratch and Orig's adjoint, the boundary split in three,
 // slopes^T by faces, edge shares a thread each and the species' sweep adjoints
 // in a loop (220 -> 198 KB of code).
@@ -236,7 +236,6 @@ __device__ inline void bc_adjoint_upper(const ColCtx& c, const ColAdj& a, int s)
       a.x(F_LRHO, nA + 2) = 0.0;
     }
   }
-  __syncwarp();
   __syncwarp();
   // lines 420-486: species winds and hydrostatic densities, one per lane
   double tb = 0.0;
@@ -1218,8 +1217,8 @@ __global__ void __launch_bounds__(NT, 1) vert_adjoint_kernel(const AParams kp) {
       return sm + size_t(A.stride) * cl + L.X1 +
              (r < NF * 4 ? (r >> 2) * G + (u < 2 ? u : nA + u) : NF * G + r - NF * 4);
     };
-    // bc^T of every column on the state in X0 with the pre-boundary ghost
-    // values of saved state s_pre: the ions of a column, the neutrals of two,
+    // bc^T of every column on the state in X0 (pg1, pg2: the pre-boundary ions
+    // of this thread's column at nAlts+1 and nAlts+2): the ions of a column, the neutrals of two,
     // each a warp's task; the two ends of a column in turn where they meet
     auto boundaries_adjoint = [&](double pg1, double pg2) {
       const int np = (nc + 1) / 2;  // pairs of columns (nc <= nw: the ions are a warp's first task)

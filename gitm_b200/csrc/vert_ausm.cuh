@@ -85,7 +85,8 @@ __device__ __forceinline__ void ausm_prefix(ColCtx c, int lane) {
 // the 4th-order form of the last five (2nd-order at cells 0 and nAlts+1).  A
 // species' values are read once for its density and pressure slopes, and the
 // grid's coefficients once for all, ahead of the stores they would otherwise
-// be read again after (2.5 degrees, 4 steps: 6.94 -> 5.96 ms).
+// be read again after (2.5 degrees, 4 steps: 6.94 -> 5.96 ms; 6.09 with the
+// warps brought together at every tensor-memory access).
 __device__ __forceinline__ void ausm_slopes_cell(ColCtx c, int i, double beta) {
   const int nA = c.L.nAlts;
   const double id1 = c.g(GC_IDF, i + 1), id0 = c.g(GC_IDF, i);

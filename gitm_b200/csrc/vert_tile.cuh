@@ -15,10 +15,10 @@
 //      P  set_vertical_bcs on every column and the limited slopes
 //      B  advance_vertical_1stage at every cell, increments to tensor memory
 //      C  the RK combination, each thread its own cell
-//  * P is a queue of warp-sized tasks: the upper boundary of three columns
-//    (lanes over ions), the lower boundary of five (lanes over species),
-//    each with the slopes next to its ghost cells, and the slopes of 32
-//    (field, run of about 16 cells) pairs.  The boundary chains, which kept
+//  * P is a queue of warp-sized tasks: the ions' boundaries of three columns
+//    (lanes over ions), the upper boundary of two and the lower boundary of two
+//    (lanes over species), each with the slopes next to its ghost cells, and
+//    the slopes of 32 (field, run of about 16 cells) pairs.  The boundary chains, which kept
 //    every warp busy for a fifth of the step, run beside the slopes.  A run
 //    slides along its cells: one load and one difference per slope instead
 //    of five and two.
@@ -36,7 +36,7 @@
 // 56.3 with the LDL^T friction, 48.2 with tensor memory, 10 columns and the
 // task queue, 41.8 with single copies of the code and the batched exp / log,
 // 38.5 with the conflict-free column stride.  Uneven ensemble (nAlts 50 / 75 /
-// 100, 2 steps): 11.1 -> 7.04 ms.
+// 100, 2 steps): 11.1 -> 7.06 ms.
 #pragma once
 
 #include "vert_kernel.cuh"

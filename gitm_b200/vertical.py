@@ -181,6 +181,9 @@ class Plan:
         return c
 
     def set_config(self, threads=256, cols_per_cta=0, steps_per_launch=1, ctas_per_sm=0):
+        """gitm_vert_plan_set_config.  Every field is set: without `threads` the
+        plan takes the 256-thread shape, whatever it had (a new Rusanov plan has
+        512, the faster one; autotune() picks the fastest)."""
         c = abi.GitmLaunchConfig(threads, cols_per_cta, steps_per_launch, ctas_per_sm)
         _check(lib().gitm_vert_plan_set_config(self.handle, C.byref(c)), self.ctx.handle, "set_config")
 

@@ -121,6 +121,9 @@ typedef struct GitmVertParams {
  *   velocity   [3]  Velocity (E,N,Up)  vert_vel   [6]  VerticalVelocity
  * Optional outputs (may be NULL):
  *   log_ns     [6]  LogNS              ndensity        NDensity
+ *     (formed by the step, so not for a column it refuses, whose density is not
+ *     positive: device arrays keep what they held there; the calls that stage
+ *     their arrays, _native_host and _fortran, give zeros)
  * Coefficients, one field each (read; written when compute_coefficients=1,
  * in which case they may be NULL):
  *   gamma (Gamma), mean_major_mass (MeanMajorMass), temp_unit (TempUnit),
