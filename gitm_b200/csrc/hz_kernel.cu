@@ -47,6 +47,16 @@ constexpr int HZ_NGP = 6;   // metric planes with ghost rings: IFB, DFB lon; IFB
 constexpr int HZ_NLD = HZ_NSW + 4;  // planes loaded whole: the fields and the four metrics
 constexpr int HZ_PER = 5;   // fields of a thread
 constexpr int HZ_GRP = 4;   // threads of a cell: fields 5 g .. 5 g + 4
+// A thread takes a line's slopes of up to HZ_LINE cells, HZ_PART of a longer
+// one: a line of 128 cells was one thread's chain while the CTA waited (40
+// blocks of 128 x 2 cells at 20 altitudes 1,977 us, now 493; 770 with a thread
+// per cell).  Parts of 5, 7, 8 and 9 cells, 30 blocks at 10 altitudes: 128 x 2
+// 249, 250, 249 and 252 us (343 with a thread per cell), 100 x 2 268, 273, 292
+// and 291 (285), 42 x 2 105, 105, 121 and 119 (150): an odd length keeps the
+// parts' lanes on different banks.  Ordinary lines stay whole, in instances of
+// their own: the parts' index arithmetic cost 9 x 9 blocks 6 %.
+constexpr int HZ_LINE = 26;
+constexpr int HZ_PART = 5;
 constexpr double F1 = 0.6250000;  // Factor1, advance_horizontal.f90:939
 constexpr double F2 = 0.0416667;  // Factor2, advance_horizontal.f90:940
 static_assert(HZ_PER * HZ_GRP >= HZ_NSW && HF_N == HZ_PER, "the groups' fields");
@@ -85,18 +95,24 @@ __host__ __device__ inline HzLayout hz_layout(int nLons, int nLats, int batch, b
   return L;
 }
 
-// The limited slopes of one line (calc_facevalues_lons / _lats): cells 0 ..
-// n+1 of values V and inverse face distances IF, both with stride s (index 0
-// = cell -1), to d with stride sd.  4th-order differences, with the 2nd-order
-// one on the outer side of cells 0 and n+1.  Along the line each value and
-// each difference is formed once: 3 shared-memory accesses and 11 FP64
-// instructions per slope (9 and 16 with a thread per slope).
-__device__ __forceinline__ void hz_slopes(const double* V, const double* IF, double* d, int s, int sd, int n,
-                                          double beta) {
-  double vm = V[0], v0 = V[s], vp = V[2 * s];  // cells -1, 0, 1
-  double dn = (v0 - vm) * IF[s];               // between cells -1 and 0: 2nd order
+// The limited slopes of cells q0 .. q1 of one line (calc_facevalues_lons /
+// _lats; cells 0 .. n+1) of values V and inverse face distances IF, both with
+// stride s (index 0 = cell -1), to d with stride sd.  4th-order differences,
+// with the 2nd-order one on the outer side of cells 0 and n+1.  Along the line
+// each value and each difference is formed once: 3 shared-memory accesses and
+// 11 FP64 instructions per slope (9 and 16 with a thread per slope).
+__device__ __forceinline__ void hz_slopes(const double* V, const double* IF, double* d, int s, int sd, int q0, int q1,
+                                          int n, double beta) {
+  double vm = V[q0 * s], v0 = V[(q0 + 1) * s], vp = V[(q0 + 2) * s];  // cells q0-1, q0, q0+1
+  // between cells q0-1 and q0; of cell 0 the 2nd-order one
+  double dn = IF[(q0 + 1) * s];
+  if (q0 == 0)
+    dn = (v0 - vm) * dn;
+  else
+    dn = (dn * 2) * (F1 * (v0 - vm) - F2 * (vp - V[(q0 - 1) * s]));
+  const int last = min(q1, n);
 #pragma unroll 4
-  for (int q = 0; q <= n; ++q) {
+  for (int q = q0; q <= last; ++q) {
     // between cells q and q+1
     const double vq = V[(q + 3) * s];
     const double up = (IF[(q + 2) * s] * 2) * (F1 * (vp - v0) - F2 * (vq - vm));
@@ -106,7 +122,7 @@ __device__ __forceinline__ void hz_slopes(const double* V, const double* IF, dou
     v0 = vp;
     vp = vq;
   }
-  d[(n + 1) * sd] = limiter_mc((vp - v0) * IF[(n + 3) * s], dn, beta);
+  if (q1 > n) d[(n + 1) * sd] = limiter_mc((vp - v0) * IF[(n + 3) * s], dn, beta);
 }
 
 // A cell's faces along one direction: halves of the face widths, the
@@ -134,12 +150,14 @@ struct HzArgs {
   uint32_t* status;  // one word per block
   int group;         // threads of a field group: the interior cells rounded up to whole warps
   int batch;         // see hz_layout
-  unsigned magic;    // ceil(2^32 / lines of a field): w / lines = umulhi(w, magic) for w < 2^16
+  int parts_lon, parts_lat;  // threads that share a line (1, or parts of HZ_PART cells)
+  unsigned magic;    // ceil(2^32 / tasks of a field): w / tasks = umulhi(w, magic) for w < 2^16
 };
 
 // Threads: HZ_GRP groups of A.group (at most NT in all); thread q of a group
-// has interior cell q.
-template <int NT, int MINB, bool KEEP>
+// has interior cell q.  SPLIT: lines of more than HZ_LINE cells are shared by
+// threads.
+template <int NT, int MINB, bool KEEP, bool SPLIT>
 __global__ void __launch_bounds__(NT, MINB) hz_step_kernel(const HzArgs A) {
   extern __shared__ double sm[];
   const GitmHzBlocks& B = A.b;
@@ -255,7 +273,7 @@ __global__ void __launch_bounds__(NT, MINB) hz_step_kernel(const HzArgs A) {
   auto value = [&](int m) { return KEEP ? sm[L.M + m * L.C + q] : other(m)[pg]; };
   // where the cell's slopes stand in a field's slope row
   const int dl = (cj - 1) * L.NLp + ci, dt0 = L.NL + cj * nl + (ci - 1);
-  const int per = L.per, lines = nl + nt;
+  const int per = L.per, lines = SPLIT ? nt * A.parts_lon + nl * A.parts_lat : nl + nt;
   auto sweeps = [&](int f, int fb, double& gLo, double& gLa, double& dd) {
     const double* v = S + f * P + pc;
     const double* d = D + (f - fb) * per;
@@ -273,15 +291,24 @@ __global__ void __launch_bounds__(NT, MINB) hz_step_kernel(const HzArgs A) {
     for (int j = 0; j < HZ_PER; ++j) kv[j] = 0.0;
 #pragma unroll 1
     for (int fb = 0; fb < HZ_NSW; fb += A.batch) {
-      // slopes, a line of a field per thread
+      // slopes, a line of a field per thread, or a part of one where lines are long
       const int n = (min(fb + A.batch, HZ_NSW) - fb) * lines;
       for (int w = tid; w < n; w += nthr) {
         const int f = __umulhi(unsigned(w), A.magic), r = w - f * lines;
-        const bool lat = r >= nt;
-        const int x = lat ? r - nt : r;  // row x + 1, or column x + 1
+        const int lons = SPLIT ? nt * A.parts_lon : nt;
+        const bool lat = r >= lons;
+        const int len = lat ? nt : nl;
+        int x = lat ? r - lons : r;  // row x + 1, or column x + 1
+        int q0 = 0, q1 = len + 1;
+        if (SPLIT && (lat ? A.parts_lat : A.parts_lon) > 1) {
+          const int across = lat ? nl : nt, part = x / across;
+          x -= part * across;
+          q0 = part * HZ_PART;
+          q1 = min(q0 + HZ_PART - 1, q1);
+        }
         const int at = lat ? x + 2 : (x + 2) * NI;
         hz_slopes(S + (fb + f) * P + at, GP + (lat ? 2 * P : 0) + at, D + f * per + (lat ? L.NL + x : x * L.NLp),
-                  lat ? NI : 1, lat ? nl : 1, lat ? nt : nl, beta);
+                  lat ? NI : 1, lat ? nl : 1, q0, q1, len, beta);
       }
       __syncthreads();
       // cells
@@ -605,9 +632,20 @@ size_t hz_smem_bytes(int n_lons, int n_lats) {
   return hz_smem(n_lons, n_lats, hz_batch(n_lons, n_lats), hz_keep(n_lons, n_lats));
 }
 
+// Threads for the slopes of a line of n cells.
+static int hz_parts(int n) { return n + 2 <= HZ_LINE ? 1 : (n + 2 + HZ_PART - 1) / HZ_PART; }
+
 int hz_threads(int n_lons, int n_lats) {
   const int c = n_lons * n_lats;
   return c <= 256 ? HZ_GRP * ((c + 31) / 32 * 32) : 0;
+}
+
+template <bool SPLIT>
+static const void* hz_kernel(int threads, bool keep) {
+  if (!keep) return (const void*)hz_step_kernel<1024, 1, false, SPLIT>;
+  return threads <= 384   ? (const void*)hz_step_kernel<384, 2, true, SPLIT>
+         : threads <= 768 ? (const void*)hz_step_kernel<768, 1, true, SPLIT>
+                          : (const void*)hz_step_kernel<1024, 1, true, SPLIT>;
 }
 
 cudaError_t hz_launch(const GitmHzParams& prm, const GitmHzBlocks& b, double dt, uint32_t* status,
@@ -620,13 +658,14 @@ cudaError_t hz_launch(const GitmHzParams& prm, const GitmHzBlocks& b, double dt,
   const int nt = hz_threads(b.n_lons, b.n_lats);
   a.group = nt / HZ_GRP;
   a.batch = hz_batch(b.n_lons, b.n_lats);
-  a.magic = unsigned(((uint64_t(1) << 32) + (b.n_lons + b.n_lats) - 1) / (b.n_lons + b.n_lats));
+  a.parts_lon = hz_parts(b.n_lons);
+  a.parts_lat = hz_parts(b.n_lats);
+  const unsigned tasks = unsigned(b.n_lats * a.parts_lon + b.n_lons * a.parts_lat);
+  a.magic = unsigned(((uint64_t(1) << 32) + tasks - 1) / tasks);
   const size_t smem = hz_smem_bytes(b.n_lons, b.n_lats);
   // up to 96 cells (9 x 9 blocks, GITM's usual size): two CTAs or more per SM
   const bool keep = hz_keep(b.n_lons, b.n_lats);
-  const void* fn = keep ? (nt <= 384   ? (const void*)hz_step_kernel<384, 2, true>
-                           : nt <= 768 ? (const void*)hz_step_kernel<768, 1, true> : (const void*)hz_step_kernel<1024, 1, true>)
-                        : (const void*)hz_step_kernel<1024, 1, false>;
+  const void* fn = (a.parts_lon > 1 || a.parts_lat > 1) ? hz_kernel<true>(nt, keep) : hz_kernel<false>(nt, keep);
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
   if (e != cudaSuccess) return e;
   void* args[] = {&a};
