@@ -868,12 +868,15 @@ static int adjoint_chunks(GitmVertPlan* P) {
   for (;;) {
     std::vector<AdjChunk> cut = adjoint_cut(P->save_tiles, P->adj_tiles, n_cols, columns);
     const int64_t most = adjoint_cut_largest(cut);
-    if (most != last &&
-        plan_alloc(P, &P->d_adj_states, size_t(ADJ_NSTATE) * most * P->adj_per_max) == cudaSuccess) {
-      P->adj_chunks = std::move(cut);
-      return GITM_OK;
+    if (most != last) {
+      const cudaError_t e = plan_alloc(P, &P->d_adj_states, size_t(ADJ_NSTATE) * most * P->adj_per_max);
+      if (e == cudaSuccess) {
+        P->adj_chunks = std::move(cut);
+        return GITM_OK;
+      }
+      if (e != cudaErrorMemoryAllocation) CUDA_TRY(ctx, e);  // under a capture, say
+      cudaGetLastError();
     }
-    cudaGetLastError();
     if (columns <= 1)
       return set_err(ctx, GITM_ERR_NOMEM, "adjoint: cannot allocate the stage states of %lld columns", (long long)most);
     last = most;

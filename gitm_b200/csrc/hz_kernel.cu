@@ -49,7 +49,7 @@ constexpr int HZ_PER = 5;   // fields of a thread
 constexpr int HZ_GRP = 4;   // threads of a cell: fields 5 g .. 5 g + 4
 // A thread takes a line's slopes of up to HZ_LINE cells, HZ_PART of a longer
 // one: a line of 128 cells was one thread's chain while the CTA waited (40
-// blocks of 128 x 2 cells at 20 altitudes 1,977 us, now 493; 770 with a thread
+// blocks of 128 x 2 cells at 20 altitudes 1,977 us, now 499; 770 with a thread
 // per cell).  Parts of 5, 7, 8 and 9 cells, 30 blocks at 10 altitudes: 128 x 2
 // 249, 250, 249 and 252 us (343 with a thread per cell), 100 x 2 268, 273, 292
 // and 291 (285), 42 x 2 105, 105, 121 and 119 (150): an odd length keeps the

@@ -380,7 +380,8 @@ typedef struct GitmColumnAdjoint {
  * per member, device pointers).  Supported: GITM-array plans, the Rusanov
  * solver.  Columns whose step met GITM_ST_ADJ_BRANCH set that bit in the
  * plan's status words.  saved_states: the states gitm_vert_plan_advance_saving
- * wrote for this step, or NULL to have the saving step run ahead of the adjoint kernel.
+ * wrote for this step, or NULL to have the saving step run ahead of the adjoint kernel
+ * (the first such call takes the buffer for its states: make it before a capture).
  * Asynchronous on `stream` (the descriptors are read before the call
  * returns). */
 int gitm_vert_plan_adjoint(GitmVertPlan* plan, const GitmColumnAdjoint* bars, double dt,
