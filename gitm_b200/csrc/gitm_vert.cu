@@ -1298,14 +1298,20 @@ extern "C" int gitm_vert_advance_native_host(GitmVertCtx* ctx, const GitmColumnB
     return GITM_OK;
   };
   // A chunk's copies out go after the copies in of the chunk behind it, where
-  // there are four chunks or more.  Right behind the step they cross with the
-  // copies in, which they slow down more than they gain, and the more so the
-  // sooner the step is done: with the steps 1.15 times as fast the call had
-  // become up to 6 % slower.  8,920 columns of 90 altitudes 5.89 -> 5.23 ms,
-  // 10,368 of 50 4.11 -> 3.71, 30,000 of 50 11.7 -> 9.4; two chunks behind 5.58,
-  // 3.90, 9.8; up to three chunks there is too little to cross (2,592 columns of
-  // 50 1.27 ms without, 1.30 with).
-  const size_t lag = chunks.size() >= 4 ? 1 : 0;
+  // there are four chunks or more and a chunk's rows are no longer than 16 KB.
+  // Right behind the step they cross with the copies in, which they slow down
+  // more than they gain, and the more so the sooner the step is done: with the
+  // steps 1.15 times as fast the call had become up to 6 % slower.  8,920
+  // columns of 90 altitudes 5.89 -> 5.23 ms, 10,368 of 50 4.11 -> 3.71, 30,000 of
+  // 50 (rows of 15 KB) 12.0 -> 9.6; two chunks behind 5.58, 3.90, 9.8.  Up to
+  // three chunks there is too little to cross (2,592 columns of 50 1.27 ms at
+  // once, 1.30 one behind), and longer rows cross well: 36,000 columns of 50
+  // 10.8 ms at once, 11.1 one behind, 64,800 of 50 22.0 and 21.6, with LogNS and
+  // NDensity 24.8 and 25.5, 64,800 of 100 39.5 and 40.4.
+  constexpr int64_t kLagCols = 2048;
+  int64_t widest = 0;
+  for (const Chunk& ch : chunks) widest = std::max(widest, ch.n);
+  const size_t lag = chunks.size() >= 4 && widest <= kLagCols ? 1 : 0;
   for (size_t j = 0; j < chunks.size() && !rc; ++j) {
     const Chunk& ch = chunks[j];
     const GitmColumnBatch& b = members[ch.m];
@@ -1332,9 +1338,11 @@ extern "C" int gitm_vert_advance_native_host(GitmVertCtx* ctx, const GitmColumnB
       if ((rc = h2d(const_cast<double*>(d.*(a.field)), b.*(a.field), rows_of(a.rows_per_cell, G)))) break;
     }
     if (rc) break;
-    // formed by the step alone, and not for a column it refuses: the copies out give such a column zeros
+    // formed by the step alone, and not for a column it refuses: the copies out give such a column
+    // zeros.  On the steps' stream: between the copies in they cost 1 % of a call (16,000 columns
+    // of 50 altitudes with both 6.30 -> 6.14 ms)
     for (double* p : {d.log_ns, d.ndensity})
-      if (p) CUDA_TRY(ctx, cudaMemsetAsync(p, 0, size_t(p == d.log_ns ? NS : 1) * G * w, s_in));
+      if (p) CUDA_TRY(ctx, cudaMemsetAsync(p, 0, size_t(p == d.log_ns ? NS : 1) * G * w, s_k));
     CUDA_TRY(ctx, cudaEventRecord(e_in, s_in));
     CUDA_TRY(ctx, cudaStreamWaitEvent(s_k, e_in, 0));
     const int spl = std::max(1, P->cfg.steps_per_launch);

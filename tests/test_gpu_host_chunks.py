@@ -27,3 +27,16 @@ def test_chunks(shape):
             for k in STATE:
                 np.testing.assert_array_equal(getattr(h, k), w[k], err_msg=k)
     ctx.close()
+
+
+@pytest.mark.parametrize("n", [32768, 32784])  # chunks of 2,048 and 2,049 columns: either order of the copies
+def test_long_rows(n):
+    p = abi.default_params()
+    m = synthetic.make_member(n, 8, seed=47)
+    want = gpu_advance(m, p, 2.0, config=dict(threads=128, steps_per_launch=1))[0]
+    ctx = V.VerticalContext(p)
+    h = m.copy()
+    V.advance_vertical_all_host(ctx, [h], 2.0)
+    for k in STATE:
+        np.testing.assert_array_equal(getattr(h, k), want[k], err_msg=k)
+    ctx.close()
